@@ -29,9 +29,8 @@ namespace {
 #endif
 constexpr int kBins = SHB_BVH_BINS;
 constexpr int kMaxLeaf = SHB_BVH_MAX_LEAF;  // triangles per leaf child of a wide node
-// A wide node's triangle group is a 24-bit mask (bit 31 marks node groups in
-// the traversal), so its 8 leaf children hold at most 24 triangles.
-static_assert(kMaxLeaf >= 1 && kMaxLeaf * 8 <= 24, "leaf triangles must fit the 24-bit triangle group");
+// A wide node's mask has three triangle bits per slot.
+static_assert(kMaxLeaf >= 1 && kMaxLeaf <= 3, "a leaf slot holds at most three triangles");
 constexpr int kMaxDepth = 40;  // deeper nodes use median splits
 constexpr int kThreads = 256;
 
@@ -561,10 +560,6 @@ __global__ void k_collapse(int n_level, const int* __restrict__ level, const BNo
   }
 }
 
-__device__ __forceinline__ uint32_t set_byte(uint32_t word, int k, uint32_t v) {
-  return (word & ~(0xFFu << (8 * k))) | ((v & 0xFFu) << (8 * k));
-}
-
 __global__ void k_emit(int n_level, int wide_base, int child_wide_base, int tri_base_all,
                        const Collapse* __restrict__ col, const int* __restrict__ int_off, const int* __restrict__ tri_off,
                        const BNode* __restrict__ nodes, const uint32_t* __restrict__ idx,
@@ -596,8 +591,9 @@ __global__ void k_emit(int n_level, int wide_base, int child_wide_base, int tri_
       ebits |= (uint32_t)(e + 127) << (8 * a);
       scale[a] = __int_as_float((e + 127) << 23);
     }
-    uint32_t imask = 0, meta_lo = 0, meta_hi = 0;
-    uint32_t qlo[6] = {0, 0, 0, 0, 0, 0}, qhi[6] = {0, 0, 0, 0, 0, 0};
+    uint32_t mask = 0;
+    for (int a = 0; a < 6; ++a)
+      for (int s = 0; s < 8; ++s) nd.q[a][s] = 0;
     int child_base = child_wide_base + int_off[w];
     int tri_base = tri_base_all + tri_off[w];
     int r_int = 0, t_off = 0;
@@ -606,14 +602,12 @@ __global__ void k_emit(int n_level, int wide_base, int child_wide_base, int tri_
       int b = by_slot[s];
       if (b < 0) continue;
       const BNode& ch = nodes[b];
-      uint32_t meta;
       if (!((leaf_slots >> s) & 1u)) {
-        imask |= 1u << s;
-        meta = (1u << 5) | (24u + (uint32_t)s);  // one bit at 24 + slot (see WideNode)
+        mask |= 1u << s;
         next_level[int_off[w] + r_int] = b;
         r_int++;
       } else {
-        meta = ((uint32_t)ch.count << 5) | (uint32_t)t_off;
+        for (int k = 0; k < ch.count; ++k) mask |= 0x80000000u >> (3 * s + k);
         for (int k = 0; k < ch.count; ++k) {
           uint32_t prim = idx[ch.begin + k];
           int64_t o = 3 * (int64_t)(tri_base + t_off + k);
@@ -625,8 +619,6 @@ __global__ void k_emit(int n_level, int wide_base, int child_wide_base, int tri_
         }
         t_off += ch.count;
       }
-      if (s < 4) meta_lo = set_byte(meta_lo, s, meta);
-      else meta_hi = set_byte(meta_hi, s - 4, meta);
       for (int a = 0; a < 3; ++a) {
         float l = floorf(__fdiv_rd(__fsub_rd(ch.lo[a], p[a]), scale[a]));
         float h = ceilf(__fdiv_ru(__fsub_ru(ch.hi[a], p[a]), scale[a]));
@@ -634,20 +626,15 @@ __global__ void k_emit(int n_level, int wide_base, int child_wide_base, int tri_
         int qh = h < 0.f ? 0 : (h > 255.f ? 255 : (int)h);
         while (ql > 0 && __fadd_rn(p[a], __fmul_rn((float)ql, scale[a])) > ch.lo[a]) ql--;
         while (qh < 255 && __fadd_rn(p[a], __fmul_rn((float)qh, scale[a])) < ch.hi[a]) qh++;
-        int word = a * 2 + (s >> 2);
-        qlo[word] = set_byte(qlo[word], s & 3, (uint32_t)ql);
-        qhi[word] = set_byte(qhi[word], s & 3, (uint32_t)qh);
+        nd.q[a][s] = (uint8_t)ql;
+        nd.q[3 + a][s] = (uint8_t)qh;
       }
     }
-    nd.e_imask = ebits | (imask << 24);
+    nd.exps = ebits;
     nd.child_base = (uint32_t)child_base;
     nd.tri_base = (uint32_t)tri_base;
-    nd.meta_lo = meta_lo;
-    nd.meta_hi = meta_hi;
-    for (int k = 0; k < 6; ++k) {
-      nd.qlo[k] = qlo[k];
-      nd.qhi[k] = qhi[k];
-    }
+    nd.mask = mask;
+    nd.pad = 0;
     wide[wide_base + w] = nd;
   }
 }

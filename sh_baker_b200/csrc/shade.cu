@@ -1295,7 +1295,8 @@ shb_status find_occlusion_device(shb_scene* s, const shb_ray* d_rays, int64_t n,
   int* cnt = c->counters.as<int>();
   SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_COUNT, c->stream));
   float4* hits = c->scratch[9].as<float4>();
-  launch_closest_rays(c->stream, s->bvh(), d_rays, n, hits, cnt + CNT_ERROR);
+  launch_closest_rays(c->stream, traversal_grid(c->device, false), s->bvh(), d_rays, n, hits, cnt + CNT_FETCH_EXT,
+                      cnt + CNT_ERROR);
   k_occ_attrs<<<grid_for(n), kThreads, 0, c->stream>>>(s->view(), d_rays, hits, n, d_hits);
   count_launch(c, 2);
   SHB_CUDA(cudaGetLastError());
@@ -1597,8 +1598,8 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
     a.n_tex = w.n_tex;
     const bool split_nee = splits(w);
     // traversal of a one-bake wave skips the per-ray bake lookup
-    const BakeItem* bk = w.bake >= 0 ? d_items + w.bake : d_items;
-    const int nbk = w.bake >= 0 ? 1 : nb;
+    const int only = w.bake >= 0 ? w.bake : (nb == 1 ? 0 : -1);
+    const BvhView* one = only >= 0 ? &items[only].bvh : nullptr;
     cudaMemsetAsync(cnt, 0, sizeof(int) * (CNT_FETCH_SHADOW + 1), st);
     Pair pg = stamp(2);
     a.one_bake = w.bake;
@@ -1611,7 +1612,7 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
       cudaMemsetAsync(cnt + nxt, 0, sizeof(int), st);
       cudaMemsetAsync(cnt + CNT_FETCH_EXT, 0, sizeof(int) * 2, st);
       Pair pe = stamp(0);
-      launch_extend(st, tgrid, bk, nbk, a.info, a.ext[cur], cnt + cur, a.ext_cap, a.hits, cnt + CNT_FETCH_EXT,
+      launch_extend(st, tgrid, one, d_items, a.info, a.ext[cur], cnt + cur, a.ext_cap, a.hits, cnt + CNT_FETCH_EXT,
                     cnt + CNT_ERROR, c64, prm.max_iters);
       close_stamp(pe);
       Pair pd = stamp(2);
@@ -1627,7 +1628,7 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
       }
       close_stamp(pd);
       Pair ps = stamp(1);
-      launch_shadow(st, tgrid_sh, bk, nbk, a.sh, cnt + CNT_SHADOW, a.sh_cap, a.path_L, a.nee_li, a.pend,
+      launch_shadow(st, tgrid_sh, one, d_items, a.sh, cnt + CNT_SHADOW, a.sh_cap, a.path_L, a.nee_li, a.pend,
                     cnt + CNT_FETCH_SHADOW, cnt + CNT_ERROR, c64, prm.max_iters);
       close_stamp(ps);
       if (bwd) {

@@ -197,20 +197,16 @@ struct DLight {
 // axis a), so a ray visits slots in order i ^ octant(ray).
 struct alignas(16) WideNode {
   float px, py, pz;
-  uint32_t e_imask;   // ex | ey<<8 | ez<<16 | imask<<24
-  uint32_t child_base;
-  uint32_t tri_base;
-  uint32_t meta_lo;   // meta of slots 0..3 (byte each)
-  uint32_t meta_hi;   // meta of slots 4..7
-  uint32_t qlo[6];    // qlo_x[8], qlo_y[8], qlo_z[8]
-  uint32_t qhi[6];    // qhi_x[8], qhi_y[8], qhi_z[8]
+  uint32_t exps;        // biased exponents of the grid, ex | ey << 8 | ez << 16
+  uint32_t child_base;  // first internal child; the others follow in slot order
+  uint32_t tri_base;    // first triangle; the leaves' triangles follow in slot order
+  // What exists: bit 31 - (3 s + k) triangle k of leaf slot s (at most 3),
+  // bit s an internal child in slot s.
+  uint32_t mask;
+  uint32_t pad;
+  uint8_t q[6][8];      // planes by slot: low x, y, z, high x, y, z
 };
 static_assert(sizeof(WideNode) == 80, "WideNode must be 80 bytes");
-// meta byte = count << 5 | position: the child contributes `count` bits
-// from `position` to a node's hit mask.  Empty slot: 0.  Leaf: its
-// triangle count and its first triangle's offset from tri_base (< 24).
-// Internal child in slot s: count 1, position 24 + s (the traversal XORs s
-// with the ray octant, so the hit mask's bits 24..31 are in visiting order).
 
 struct BvhView {
   const WideNode* nodes;

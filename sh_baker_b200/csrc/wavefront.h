@@ -79,13 +79,16 @@ using PathInfo = uint4;
 // Launch helpers for the persistent traversal kernels (traverse.cu).
 // max_iters bounds the traversal steps of one ray (0: the default,
 // 2^22); a ray that reaches it sets ERR_ITER and ends.
-void launch_extend(cudaStream_t st, int grid, const BakeItem* bakes, int n_bakes, const PathInfo* info, ExtQueue q,
-                   const int* n, int cap, float4* hits, int* fetch, int* err, Counters64* stats, uint32_t max_iters);
-void launch_shadow(cudaStream_t st, int grid, const BakeItem* bakes, int n_bakes, ShadowQueue q, const int* n, int cap,
-                   float4* path_L, float4* nee_li, float4* pend, int* fetch, int* err, Counters64* stats,
+// `one`: the BVH of the one bake all rays belong to (host copy), or null:
+// each ray's bake is looked up in the device table `bakes`.
+void launch_extend(cudaStream_t st, int grid, const BvhView* one, const BakeItem* bakes, const PathInfo* info,
+                   ExtQueue q, const int* n, int cap, float4* hits, int* fetch, int* err, Counters64* stats,
                    uint32_t max_iters);
-void launch_closest_rays(cudaStream_t st, const BvhView& bvh, const shb_ray* rays, int64_t n, float4* hits,
-                         int* err);
+void launch_shadow(cudaStream_t st, int grid, const BvhView* one, const BakeItem* bakes, ShadowQueue q, const int* n,
+                   int cap, float4* path_L, float4* nee_li, float4* pend, int* fetch, int* err, Counters64* stats,
+                   uint32_t max_iters);
+void launch_closest_rays(cudaStream_t st, int grid, const BvhView& bvh, const shb_ray* rays, int64_t n, float4* hits,
+                         int* fetch, int* err);
 int traversal_grid(int device, bool shadow);
 
 }  // namespace shb
