@@ -33,7 +33,7 @@ SOURCES = {
     "atlas.cpp": [],
     "preview.cu": ["-fmad=false"],
 }
-HEADERS = ["shb_internal.h", "shb_math.cuh", "wavefront.h", "tspace.h"]
+HEADERS = ["shb_internal.h", "shb_math.cuh", "wavefront.h", "f32x2.cuh", "tspace.h"]
 
 
 def nvcc() -> str:

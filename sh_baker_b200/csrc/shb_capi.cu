@@ -173,34 +173,81 @@ void srgb_table(float out[256]) {
 
 void srgb_upload(const float table[256]);
 
-// Emission constants of the area lights (DLight::er/eg/eb, emis_const): for
-// a material whose albedo does not vary over the surface, albedo *
-// emission with the float products get_emission makes on the device.
-void area_emission_consts(shb_scene* s) {
+// Constants of the lights (DLight::er/eg/eb, emis_const, pair, grey).  Area
+// lights: for a material whose albedo does not vary over the surface, albedo
+// * emission with the float products get_emission makes on the device.
+// Point lights: intensity * color.
+void light_consts(shb_scene* s) {
+  s->negative_lights = 0;
   for (uint32_t l = 0; l < s->light_count; ++l) {
     DLight& L = s->h_lights[l];
     L.emis_const = 0;
     L.er = L.eg = L.eb = 0.f;
-    if (L.type != SHB_LIGHT_AREA) continue;
-    if (L.mat < 0 || (uint32_t)L.mat >= s->mat_count) {  // load_mat's default: no emission
-      L.emis_const = 1;
-      continue;
+    L.pair = PAIR_NONE;
+    L.grey = 0;
+    for (float c : {L.cr, L.cg, L.cb})
+      if (L.type != SHB_LIGHT_AREA && !(L.intensity * c >= 0.f)) s->negative_lights = 1;
+    if (L.type == SHB_LIGHT_POINT) {
+      L.er = L.intensity * L.cr;
+      L.eg = L.intensity * L.cg;
+      L.eb = L.intensity * L.cb;
+      L.pair = PAIR_POINT;
+    } else if (L.type == SHB_LIGHT_AREA) {
+      if (L.mat < 0 || (uint32_t)L.mat >= s->mat_count) {  // load_mat's default: no emission
+        L.emis_const = 1;
+      } else {
+        const DMat& M = s->h_mats[L.mat];
+        float a[3];
+        bool known = true;
+        if (M.use_override) {
+          for (int c = 0; c < 3; ++c) a[c] = M.override_rgb[c];
+        } else if (s->h_light_albedo_const[l]) {
+          for (int c = 0; c < 3; ++c) a[c] = s->h_light_albedo[3 * l + c];
+        } else {
+          known = false;
+        }
+        if (known) {
+          L.emis_const = 1;
+          if (M.emission > 0.0f) {
+            L.er = a[0] * M.emission;
+            L.eg = a[1] * M.emission;
+            L.eb = a[2] * M.emission;
+          }
+        }
+        const bool sampled = L.geom >= 0 && (size_t)L.geom < s->h_geoms.size() && s->h_geoms[L.geom].tri_count > 0;
+        if (sampled && known) L.pair = PAIR_AREA;
+      }
     }
-    const DMat& M = s->h_mats[L.mat];
-    float a[3];
-    if (M.use_override) {
-      for (int c = 0; c < 3; ++c) a[c] = M.override_rgb[c];
-    } else if (s->h_light_albedo_const[l]) {
-      for (int c = 0; c < 3; ++c) a[c] = s->h_light_albedo[3 * l + c];
-    } else {
-      continue;
+    // pair_weights divides these by squared distances within 2^+-60: they
+    // must be 0 or keep the quotient and its residual in range
+    for (float e : {L.er, L.eg, L.eb})
+      if (!(e == 0.f || (std::fabs(e) >= 0x1p-90f && std::fabs(e) <= 0x1p30f))) L.pair = PAIR_NONE;
+    L.grey = L.er == L.eg && L.er == L.eb;
+  }
+  s->area_kind = s->area_light_count ? AREA_SINGLE : AREA_NONE;
+  for (uint32_t l = 0; l + 1 < s->light_count; ++l)
+    if (s->h_lights[l].pair == PAIR_AREA && s->h_lights[l + 1].pair == PAIR_AREA) s->area_kind = AREA_PAIRS;
+}
+
+// Box of an area light's triangles in object space (their points are sampled
+// there), with 2e-6 of the largest coordinate added for rounding.
+static void area_box(const shb_geometry_desc* geometries, DLight& L) {
+  if (L.geom < 0) return;
+  const shb_geometry_desc& g = geometries[L.geom];
+  L.bhs = 0.f;
+  for (int a = 0; a < 3; ++a) {
+    double lo = HUGE_VAL, hi = -HUGE_VAL;
+    bool finite = true;
+    for (uint32_t i = 0; i < g.index_count / 3 * 3; ++i) {
+      const double v = g.vertices[3 * (size_t)g.indices[i] + a];
+      finite = finite && std::isfinite(v);
+      lo = v < lo ? v : lo;
+      hi = v > hi ? v : hi;
     }
-    L.emis_const = 1;
-    if (M.emission > 0.0f) {
-      L.er = a[0] * M.emission;
-      L.eg = a[1] * M.emission;
-      L.eb = a[2] * M.emission;
-    }
+    if (!finite || lo > hi) lo = -HUGE_VAL, hi = HUGE_VAL;  // never behind anything
+    L.bc[a] = std::isfinite(lo) ? (float)(0.5 * (lo + hi)) : 0.f;
+    L.bh[a] = (float)(0.5 * (hi - lo) * (1.0 + 1e-6) + 2e-6 * std::fmax(std::fabs(lo), std::fabs(hi)));
+    L.bhs += L.bh[a];
   }
 }
 
@@ -335,6 +382,7 @@ SceneView shb_scene::view() const {
   v.prim_count = prim_count;
   v.vertex_count = vertex_count;
   v.has_alpha = has_alpha;
+  v.negative_lights = negative_lights;
   return v;
 }
 
@@ -597,6 +645,7 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
         L.geom = ld.geometry_index;
         L.mat = ld.material_index;
         L.area_ord = area_ord++;
+        area_box(d->geometries, L);
       }
       lights.push_back(L);
     }
@@ -632,7 +681,7 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
           s->h_light_albedo_const[l] = 1;
         }
       }
-      area_emission_consts(s);
+      light_consts(s);
       lights = s->h_lights;
     }
     shb_status rc = SHB_OK;
@@ -978,7 +1027,7 @@ shb_status shb_scene_set_params(shb_scene* s, const float* albedo_rgb, const uin
       }
     if (light_intensity)
       for (uint32_t l = 0; l < s->light_count; ++l) s->h_lights[l].intensity = light_intensity[l];
-    if (albedo_rgb) area_emission_consts(s);  // overrides change area emission
+    light_consts(s);  // overrides change area emission, intensities point lights
     cudaStream_t st = s->ctx->stream;
     if (albedo_rgb && s->mat_count)
       SHB_CUDA(cudaMemcpyAsync(s->mats.ptr, s->h_mats.data(), sizeof(DMat) * s->mat_count, cudaMemcpyHostToDevice, st));

@@ -182,14 +182,26 @@ struct DLight {
   int32_t area_ord;  // area: ordinal among area lights (RNG slots)
   // area: emission when it is the same at every point (the material's
   // albedo is untextured, a 1x1 texture or an override), computed on the
-  // host with the device's operations; emis_const 0: look it up per sample
+  // host with the device's operations; emis_const 0: look it up per sample.
+  // point: intensity times color
   float er, eg, eb;
   int32_t emis_const;
+  // PAIR_*: next to a light of the same kind, the two are weighed together
+  // (shade.cu pair_weights); grey: er, eg and eb are equal
+  int32_t pair, grey;
+  // area: box of the light's triangles (object space, widened for the
+  // rounding of sampled points): centre, half extents and their sum
+  float bc[3], bh[3], bhs;
   // area: the light's first triangle record (shade.cu sample_area) and its
   // triangle count | has-texture-uv << 31, so a sample reads them with the
   // light instead of from a separate table
   uint32_t area_first, area_count;
 };
+
+// What area lights a scene has, for the light kernels' code: none, some, or
+// some whose weights are taken in pairs.
+enum : int { AREA_NONE = 0, AREA_SINGLE = 1, AREA_PAIRS = 2 };
+enum : int32_t { PAIR_NONE = 0, PAIR_POINT = 1, PAIR_AREA = 2 };
 
 // Compressed 8-wide BVH node (80 bytes).  Children boxes are quantised on
 // a per-node power-of-two grid anchored at p; slot s holds the child whose
@@ -231,7 +243,8 @@ struct SceneView {
   const float4* area_tris;  // 4 per area-light triangle (shade.cu sample_area)
   uint32_t geom_count, mat_count, light_count, area_light_count;
   uint32_t prim_count, vertex_count;
-  int32_t has_alpha;     // any material with 4-channel albedo
+  int32_t has_alpha;        // any material with 4-channel albedo
+  int32_t negative_lights;  // a light's intensity * color has a negative channel
 };
 
 }  // namespace shb
@@ -267,6 +280,8 @@ struct shb_scene {
   uint32_t vertex_count = 0, prim_count = 0, geom_count = 0, mat_count = 0, light_count = 0;
   uint32_t area_light_count = 0;
   int32_t has_alpha = 0;
+  int32_t negative_lights = 0;
+  int area_kind = shb::AREA_NONE;
   bool raster_ready = true;  // every geometry has normals, tangents, lightmap uvs
   std::string raster_error;
   std::vector<shb::DGeom> h_geoms;

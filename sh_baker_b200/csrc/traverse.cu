@@ -22,6 +22,7 @@
 // even though this file is compiled with FMA contraction for the box tests.
 #include <cstddef>
 
+#include "f32x2.cuh"
 #include "wavefront.h"
 
 namespace shb {
@@ -230,35 +231,14 @@ __device__ __forceinline__ uint32_t bit_mask(uint32_t pos, uint32_t width) {
   return r;
 }
 
-// Pairs of floats for the packed FP32 pipe.
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(uint64_t r) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(r));
-  return f;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // Bytes 2 h and 2 h + 1 of w (a plane of two children) as distances q s + a:
 // a byte permute builds the bit pattern 0x4B0000bb = 2^23 + bb, and the
 // packed pipe subtracts 2^23 (exact) and multiplies and adds, two children
 // an instruction.
-__device__ __forceinline__ float2 planes(uint32_t w, int h, uint64_t s, uint64_t a) {
-  const uint64_t q = pack2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | (uint32_t)(2 * h))),
+__device__ __forceinline__ float2 planes(uint32_t w, int h, f32x2 s, f32x2 a) {
+  const f32x2 q = pack2(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | (uint32_t)(2 * h))),
                            __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | (uint32_t)(2 * h + 1))));
-  return unpack2(fma2(add2(q, pack2(-8388608.0f, -8388608.0f)), s, a));
+  return unpack2(fma2(add2(q, dup2(-8388608.0f)), s, a));
 }
 
 __device__ __forceinline__ void swap2(uint32_t (&a)[2], uint32_t (&b)[2]) {
@@ -298,8 +278,8 @@ __device__ __forceinline__ void intersect_node(const BvhView& bvh, Walk& w, uint
               fsz = __uint_as_float((e >> 16) << 23) * r.iz;
   const float fax = (__uint_as_float(n0.x) - r.ox) * r.ix, fay = (__uint_as_float(n0.y) - r.oy) * r.iy,
               faz = (__uint_as_float(n0.z) - r.oz) * r.iz;
-  const uint64_t sx = pack2(fsx, fsx), sy = pack2(fsy, fsy), sz = pack2(fsz, fsz);
-  const uint64_t ax = pack2(fax, fax), ay = pack2(fay, fay), az = pack2(faz, faz);
+  const f32x2 sx = dup2(fsx), sy = dup2(fsy), sz = dup2(fsz);
+  const f32x2 ax = dup2(fax), ay = dup2(fay), az = dup2(faz);
   const float tlim = w.tmax * 1.0000004f;
   uint32_t hm = 0;
 #pragma unroll
@@ -643,7 +623,12 @@ __global__ void SHB_SHADOW_BOUNDS k_shadow(BvhView one, const BakeItem* __restri
         atomicAdd(&L->z, c.z);
       }
     } else if (w.hit) {
-      (kind == 1u ? nee_li : pend)[target] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kind == 2u) {
+        pend[target] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {  // the slots of the samples that share the ray, c.y apart
+        for (uint32_t m = __float_as_uint(c.x); m; m &= m - 1)
+          nee_li[target + (uint32_t)(__ffs((int)m) - 1) * __float_as_uint(c.y)] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
   });
 }

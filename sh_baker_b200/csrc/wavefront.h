@@ -21,8 +21,9 @@ struct ExtQueue {
 // (src/light.h:40,83,128,177).
 //   o = (origin.xyz, tfar), d = (direction.xyz, target bits),
 //   c = (contribution.xyz, kind bits): kind 0 adds c to the path radiance
-//   of `target` when unoccluded; kind 1 clears texel-NEE slot `target`
-//   when occluded; kind 2 clears pending hit-NEE slot `target` when
+//   of `target` when unoccluded; kind 1 clears, when occluded, the texel-NEE
+//   slots target + l * c.y for each bit l of c.x (both as integer bits: the
+//   samples that share the ray); kind 2 clears pending hit-NEE slot `target` when
 //   occluded (deterministic accumulation, see k_commit).
 struct ShadowQueue {
   float4* o;
