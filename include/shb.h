@@ -400,7 +400,7 @@ SHB_API shb_status shb_dilate(shb_context* ctx, int32_t kind, int32_t width,
  * with a deadline where cudaMalloc's implicit synchronisation is not
  * acceptable).  Same passes and results as shb_dilate on device pointers
  * (pixels and mask on the context's device, updated in place).  The
- * ping-pong scratch lives in one fixed 16 MiB array inside the library.
+ * scratch lives in one fixed 16 MiB array inside the library.
  * Its device address is looked up by shb_context_create, so every device
  * that has had a context holds the array from then until the process
  * exits, and this call itself neither loads code nor reserves memory.  At

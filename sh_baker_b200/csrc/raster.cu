@@ -4,6 +4,7 @@
 // and src/dilation.cpp.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <mutex>
 
 #include "shb_internal.h"
@@ -247,86 +248,192 @@ __global__ void k_validity(const shb_surface_point* __restrict__ pts, int64_t n,
     out[i] = pts[i].material_id >= 0;
 }
 
-// src/rasterizer.cpp:222-241
+// src/rasterizer.cpp:222-241, a block row per output row.
 __global__ void k_mask_down(const uint8_t* __restrict__ in, int w, int h, int s, uint8_t* __restrict__ out) {
-  int64_t n = (int64_t)w * h;
-  int stride = w * s;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int x = (int)(i % w), y = (int)(i / w);
-    uint8_t any = 0;
-    for (int sy = y * s; sy < (y + 1) * s && !any; ++sy)
-      for (int sx = x * s; sx < (x + 1) * s; ++sx)
-        if (in[(int64_t)sy * stride + sx]) {
-          any = 1;
-          break;
-        }
-    out[i] = any;
+  const int64_t stride = (int64_t)w * s;
+  for (int64_t y = blockIdx.y; y < h; y += gridDim.y) {
+    const uint8_t* row = in + y * s * stride;
+    for (int64_t x = blockIdx.x * blockDim.x + threadIdx.x; x < w; x += gridDim.x * blockDim.x) {
+      uint8_t any = 0;
+      for (int dy = 0; dy < s; ++dy)
+        for (int dx = 0; dx < s; ++dx) any |= row[dy * stride + x * s + dx] != 0;
+      out[y * w + x] = any;
+    }
   }
 }
 
-// src/baker.cpp:151-182, one thread per (output texel, channel).
-__global__ void k_downsample(const float* __restrict__ in, int in_w, int in_h, int ch, int s,
-                             float* __restrict__ out) {
-  int ow = in_w / s, oh = in_h / s;
-  int64_t n = (int64_t)ow * oh * ch;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int c = (int)(i % ch);
-    int64_t texel = i / ch;
-    int x = (int)(texel % ow), y = (int)(texel / ow);
-    float avg = 0.0f;
-    int count = 0;
-    for (int dy = 0; dy < s; ++dy)
-      for (int dx = 0; dx < s; ++dx) {
-        int sx = x * s + dx, sy = y * s + dy;
-        if (sx < in_w && sy < in_h) {
-          avg += in[((int64_t)sy * in_w + sx) * ch + c];
-          count++;
-        }
+// src/baker.cpp:151-182: one thread per (output texel, channel), a block row
+// per output row.  CH and S are the channels and the scale (0: any).  Bound
+// by HBM: every input float is read once.  With both known the S * S loads
+// of a thread are independent and in flight together and the texel index is
+// a 32-bit constant division: 3072^2 SH texels to 1024^2 in 210 us (5.4 TB/s;
+// 525 us with 64-bit divisions and a loop).
+template <int CH, int S>
+__global__ void __launch_bounds__(kThreads) k_downsample(const float* __restrict__ in, int in_w, int oh, int ow,
+                                                         int ch_, int s_, float* __restrict__ out) {
+  const int ch = CH ? CH : ch_, s = S ? S : s_;
+  const int64_t row = (int64_t)ow * ch, stride = (int64_t)in_w * ch;
+  for (int64_t y = blockIdx.y; y < oh; y += gridDim.y) {
+    const float* src = in + y * s * stride;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < row; i += (int64_t)gridDim.x * blockDim.x) {
+      const int64_t x = CH ? (int64_t)((uint32_t)i / (uint32_t)CH) : i / ch;
+      const float* p = src + x * (s * ch) + (i - x * ch);
+      float avg = 0.0f;
+      if (S) {
+        float v[S ? S * S : 1];
+#pragma unroll
+        for (int k = 0; k < S * S; ++k) v[k] = __ldg(p + (k / (S ? S : 1)) * stride + (k % (S ? S : 1)) * ch);
+#pragma unroll
+        for (int k = 0; k < S * S; ++k) avg += v[k];
+      } else {
+        for (int dy = 0; dy < s; ++dy)
+          for (int dx = 0; dx < s; ++dx) avg += p[dy * stride + (int64_t)dx * ch];
       }
-    out[i] = count > 0 ? avg * (1.f / float(count)) : 0.0f;
+      out[y * row + i] = avg * (1.f / float(s * s));
+    }
   }
 }
 
-// One dilation pass (src/dilation.cpp:25-66), one thread per (texel,
-// channel).  Pass p is skipped when pass p-1 changed nothing: from then on
-// every pass is the identity, and both ping-pong buffers hold the result.
-template <class T>
-__global__ void k_dilate(const T* __restrict__ pin, const uint8_t* __restrict__ min, T* __restrict__ pout,
-                         uint8_t* __restrict__ mout, int w, int h, int ch, int* changed, int pass) {
-  if (pass > 0 && *(volatile int*)(changed + pass - 1) == 0) return;
-  int64_t n = (int64_t)w * h * ch;
+// ------------------------------------------------------------- dilation ----
+// Dilate<T> (src/dilation.cpp:25-66) in place: a texel's label is 0 when it
+// was valid, the pass that filled it, or kUnfilled.  Pass p fills the
+// unfilled texels that have a neighbour with a label below p and reads only
+// such neighbours, whose pixels are final; a label that changes to p during
+// the pass is not below p either way.  So the pixels need no second copy,
+// and a pass reads two bytes per texel and touches the pixels only where it
+// fills: the ping-pong passes this replaces read and wrote the whole texture
+// each time (16 + 16 passes over a 1024^2 SH and a visibility texture, charts
+// on 85 % of the page: 1.9 -> 0.4 ms).
+constexpr uint16_t kUnfilled = 0xFFFFu;
+constexpr int kMaxLabel = 0xFFFE;  // passes per run of labels
+
+__global__ void k_labels(const uint8_t* __restrict__ mask, int64_t n, uint16_t* __restrict__ label) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    label[i] = mask[i] ? 0 : kUnfilled;
+}
+
+// Bit (dy + 1) * 3 + (dx + 1) for each neighbour of texel (x, y) with a
+// label below `pass`.
+__device__ __forceinline__ uint32_t filled_neighbours(const uint16_t* label, int w, int h, int x, int y, int pass) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int nx = x + k % 3 - 1, ny = y + k / 3 - 1;
+    if (k == 4 || nx < 0 || nx >= w || ny < 0 || ny >= h) continue;
+    if (label[(int64_t)ny * w + nx] < pass) m |= 1u << k;
+  }
+  return m;
+}
+
+// One pass.  Pass p is skipped when pass p - 1 filled nothing.  A warp looks
+// at 8 x 4 texels at a time, of which a straight front crosses few: with
+// several channels it fills them one after the other, a lane per channel, so
+// that a texel's floats are read and written together, and the longest such
+// chain is the pass's time (with 32 texels of a row per warp it was 20 us).
+constexpr int kTileW = kThreads / 32 * 8, kTileH = 16;
+template <class T, int CH>
+__global__ void __launch_bounds__(kThreads) k_dilate(T* __restrict__ px, uint8_t* __restrict__ mask,
+                                                     uint16_t* __restrict__ label, int w, int h, int* changed,
+                                                     int pass) {
+  if (pass > 1 && *(volatile int*)(changed + pass - 2) == 0) return;
+  const int lane = threadIdx.x & 31, lx = lane & 7, ly = lane >> 3;
   bool any = false;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    int c = (int)(i % ch);
-    int64_t idx = i / ch;
-    T v = pin[i];
-    uint8_t m = min[idx];
-    if (!m) {
-      int x = (int)(idx % w), y = (int)(idx / w);
-      T acc = T();
-      int count = 0;
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          if (dx == 0 && dy == 0) continue;
-          int nx = x + dx, ny = y + dy;
-          if (nx >= 0 && nx < w && ny >= 0 && ny < h) {
-            int64_t ni = (int64_t)ny * w + nx;
-            if (min[ni]) {
-              acc = (T)(acc + pin[ni * ch + c]);
-              count++;
+  for (int64_t y0 = blockIdx.y * (int64_t)kTileH; y0 < h; y0 += gridDim.y * (int64_t)kTileH) {
+    for (int64_t x0 = blockIdx.x * (int64_t)kTileW + (threadIdx.x >> 5) * 8; x0 < w; x0 += gridDim.x * (int64_t)kTileW) {
+      const int64_t x = x0 + lx;
+      bool open[kTileH / 4];
+#pragma unroll
+      for (int r = 0; r < kTileH / 4; ++r) {
+        const int64_t y = y0 + 4 * r + ly;
+        open[r] = x < w && y < h && label[y * w + x] == kUnfilled;
+      }
+#pragma unroll
+      for (int r = 0; r < kTileH / 4; ++r) {
+        if (!__any_sync(0xFFFFFFFFu, open[r])) continue;
+        const int64_t y = y0 + 4 * r + ly, t = y * w + x;
+        const uint32_t nb = open[r] ? filled_neighbours(label, w, h, (int)x, (int)y, pass) : 0u;
+        if (CH == 1) {
+          if (nb) {
+            T acc = T();
+            for (uint32_t m = nb; m; m &= m - 1) {
+              const int k = __ffs((int)m) - 1;
+              acc = (T)(acc + px[t + (int64_t)(k / 3 - 1) * w + (k % 3 - 1)]);
+            }
+            px[t] = (T)(acc * (1.0f / __popc(nb)));
+          }
+        } else {
+          // four texels at a time, so that their loads wait together
+          for (unsigned todo = __ballot_sync(0xFFFFFFFFu, nb != 0); todo;) {
+            constexpr int kAtOnce = 4;
+            T v[kAtOnce][9];
+            uint32_t lnb[kAtOnce];
+            int64_t lt[kAtOnce];
+#pragma unroll
+            for (int q = 0; q < kAtOnce; ++q) {
+              const int l = todo ? __ffs((int)todo) - 1 : 0;
+              lnb[q] = __shfl_sync(0xFFFFFFFFu, nb, l);
+              if (!todo) lnb[q] = 0u;
+              todo &= todo - 1;
+              lt[q] = (y0 + 4 * r + (l >> 3)) * w + x0 + (l & 7);
+#pragma unroll
+              for (int k = 0; k < 9; ++k)
+                v[q][k] = lane < CH && ((lnb[q] >> k) & 1u)
+                              ? px[(lt[q] + (int64_t)(k / 3 - 1) * w + (k % 3 - 1)) * CH + lane]
+                              : T();
+            }
+#pragma unroll
+            for (int q = 0; q < kAtOnce; ++q) {
+              T acc = T();
+#pragma unroll
+              for (int k = 0; k < 9; ++k)
+                if ((lnb[q] >> k) & 1u) acc = (T)(acc + v[q][k]);
+              if (lane < CH && lnb[q]) px[lt[q] * CH + lane] = (T)(acc * (1.0f / __popc(lnb[q])));
             }
           }
         }
-      if (count > 0) {
-        v = (T)(acc * (1.0f / count));
-        m = 1;
-        any = true;
+        if (nb) {
+          label[t] = (uint16_t)pass;
+          mask[t] = 1;
+          any = true;
+        }
       }
     }
-    pout[i] = v;
-    if (c == 0) mout[idx] = m;
   }
-  if (any) changed[pass] = 1;
+  if (any) changed[pass - 1] = 1;
+}
+
+// A grid of block rows over a w x h texture.
+inline dim3 grid_rows(int64_t w, int64_t h) {
+  const int64_t gx = std::min<int64_t>((w + kThreads - 1) / kThreads, 1024);
+  const int64_t cap = std::max<int64_t>((int64_t)sm_count() * 256 / gx, 1);
+  return dim3((unsigned)gx, (unsigned)std::min<int64_t>(std::min<int64_t>(h, cap), 65535));
+}
+
+// Runs `passes` dilation passes with n labels and min(passes, kMaxLabel)
+// flags of scratch.
+shb_status dilate_passes(shb_context* c, int kind, int w, int h, void* pixels, uint8_t* mask, int passes,
+                         uint16_t* label, int* changed) {
+  cudaStream_t st = c->stream;
+  const int64_t n = (int64_t)w * h;
+  const dim3 grid((unsigned)std::min<int64_t>(((int64_t)w + kTileW - 1) / kTileW, 4096),
+                  (unsigned)std::min<int64_t>(((int64_t)h + kTileH - 1) / kTileH, 4096));
+  for (int done = 0; done < passes;) {
+    const int run = std::min(passes - done, kMaxLabel);
+    SHB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int) * (size_t)run, st));
+    k_labels<<<grid_for(n), kThreads, 0, st>>>(mask, n, label);
+    for (int p = 1; p <= run; ++p) {
+      if (kind == SHB_DILATE_U8)
+        k_dilate<uint8_t, 1><<<grid, kThreads, 0, st>>>((uint8_t*)pixels, mask, label, w, h, changed, p);
+      else if (kind == SHB_DILATE_F32)
+        k_dilate<float, 1><<<grid, kThreads, 0, st>>>((float*)pixels, mask, label, w, h, changed, p);
+      else
+        k_dilate<float, 27><<<grid, kThreads, 0, st>>>((float*)pixels, mask, label, w, h, changed, p);
+    }
+    count_launch(c, (uint64_t)run + 1);
+    done += run;
+  }
+  SHB_CUDA(cudaGetLastError());
+  return SHB_OK;
 }
 
 }  // namespace
@@ -403,9 +510,8 @@ shb_status validity_mask_device(shb_context* c, const shb_surface_point* pts, in
 }
 
 shb_status downsample_mask_device(shb_context* c, const uint8_t* in, int w, int h, int s, uint8_t* out) {
-  int64_t n = (int64_t)w * h;
-  if (n <= 0) return SHB_OK;
-  k_mask_down<<<grid_for(n), kThreads, 0, c->stream>>>(in, w, h, s, out);
+  if ((int64_t)w * h <= 0) return SHB_OK;
+  k_mask_down<<<grid_rows(w, h), kThreads, 0, c->stream>>>(in, w, h, s, out);
   count_launch(c);
   SHB_CUDA(cudaGetLastError());
   return SHB_OK;
@@ -416,9 +522,19 @@ shb_status downsample_device(shb_context* c, const float* in, int w, int h, int 
     SHB_CUDA(cudaMemcpyAsync(out, in, sizeof(float) * (size_t)w * h * ch, cudaMemcpyDeviceToDevice, c->stream));
     return SHB_OK;
   }
-  int64_t n = (int64_t)(w / s) * (h / s) * ch;
-  if (n <= 0) return SHB_OK;
-  k_downsample<<<grid_for(n), kThreads, 0, c->stream>>>(in, w, h, ch, s, out);
+  const int ow = w / s, oh = h / s;
+  if ((int64_t)ow * oh * ch <= 0) return SHB_OK;
+  const dim3 grid = grid_rows((int64_t)ow * ch, oh);
+  auto run = [&](auto kernel) { kernel<<<grid, kThreads, 0, c->stream>>>(in, w, oh, ow, ch, s, out); };
+  // (the constant division is in 32 bits)
+  if ((int64_t)ow * ch > 0xFFFFFFFFll) run(k_downsample<0, 0>);
+  else if (ch == 27 && s == 2) run(k_downsample<27, 2>);
+  else if (ch == 27 && s == 3) run(k_downsample<27, 3>);
+  else if (ch == 27 && s == 4) run(k_downsample<27, 4>);
+  else if (ch == 1 && s == 2) run(k_downsample<1, 2>);
+  else if (ch == 1 && s == 3) run(k_downsample<1, 3>);
+  else if (ch == 1 && s == 4) run(k_downsample<1, 4>);
+  else run(k_downsample<0, 0>);
   count_launch(c);
   SHB_CUDA(cudaGetLastError());
   return SHB_OK;
@@ -427,33 +543,9 @@ shb_status downsample_device(shb_context* c, const float* in, int w, int h, int 
 shb_status dilate_device(shb_context* c, int kind, int w, int h, void* pixels, uint8_t* mask, int passes) {
   int64_t n = (int64_t)w * h;
   if (n <= 0 || passes <= 0) return SHB_OK;
-  int ch = kind == SHB_DILATE_SH9 ? 27 : 1;
-  size_t esz = kind == SHB_DILATE_U8 ? 1 : 4;
-  size_t pbytes = esz * (size_t)n * ch;
-  SHB_TRY(c->scratch[6].reserve(pbytes));
-  SHB_TRY(c->scratch[7].reserve((size_t)n));
-  SHB_TRY(c->scratch[8].reserve(sizeof(int) * (size_t)passes));
-  int* changed = c->scratch[8].as<int>();
-  SHB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int) * (size_t)passes, c->stream));
-  void* bufs[2] = {pixels, c->scratch[6].ptr};
-  uint8_t* masks[2] = {mask, c->scratch[7].as<uint8_t>()};
-  int64_t work = n * ch;
-  for (int p = 0; p < passes; ++p) {
-    int src = p & 1, dst = src ^ 1;
-    if (kind == SHB_DILATE_U8)
-      k_dilate<uint8_t><<<grid_for(work), kThreads, 0, c->stream>>>(
-          (const uint8_t*)bufs[src], masks[src], (uint8_t*)bufs[dst], masks[dst], w, h, ch, changed, p);
-    else
-      k_dilate<float><<<grid_for(work), kThreads, 0, c->stream>>>(
-          (const float*)bufs[src], masks[src], (float*)bufs[dst], masks[dst], w, h, ch, changed, p);
-    count_launch(c);
-  }
-  if (passes & 1) {
-    SHB_CUDA(cudaMemcpyAsync(pixels, bufs[1], pbytes, cudaMemcpyDeviceToDevice, c->stream));
-    SHB_CUDA(cudaMemcpyAsync(mask, masks[1], (size_t)n, cudaMemcpyDeviceToDevice, c->stream));
-  }
-  SHB_CUDA(cudaGetLastError());
-  return SHB_OK;
+  SHB_TRY(c->scratch[7].reserve(sizeof(uint16_t) * (size_t)n));
+  SHB_TRY(c->scratch[8].reserve(sizeof(int) * (size_t)std::min(passes, kMaxLabel)));
+  return dilate_passes(c, kind, w, h, pixels, mask, passes, c->scratch[7].as<uint16_t>(), c->scratch[8].as<int>());
 }
 
 }  // namespace shb
@@ -466,8 +558,9 @@ shb_status dilate_device(shb_context* c, int kind, int w, int h, void* pixels, u
 // and callers on a deadline path, where cudaMalloc's implicit device-wide
 // synchronisation and unpredictable latency are not acceptable.  For them
 // shb_dilate_noalloc runs the same dilation passes as shb_dilate, but the
-// ping-pong copy of the pixels and mask and the per-pass change flags live
-// in the fixed array below.  Its device address is looked up when a
+// texels' labels and the per-pass change flags live in the fixed array
+// below.  (What it takes is bounded by a copy of pixels and mask, which the
+// array once held.)  Its device address is looked up when a
 // context is created on a device (noalloc_prepare), so the array is held on
 // every device that has had a context, from then until the process exits.
 
@@ -552,31 +645,8 @@ extern "C" SHB_API shb_status shb_dilate_noalloc(shb_context* ctx, int32_t kind,
     SHB_ON_DEVICE(ctx->device);
     unsigned char* base = nullptr;
     SHB_TRY(noalloc_scratch(ctx->device, &base));
-    int* changed = reinterpret_cast<int*>(base);
-    void* pbuf = base + kNoAllocFlagBytes;
-    uint8_t* mbuf = base + kNoAllocFlagBytes + pbytes_aligned;
-    cudaStream_t st = ctx->stream;
-    // the array keeps the previous call's contents: the change flags must start at zero
-    SHB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int) * (size_t)passes, st));
-    void* bufs[2] = {pixels, pbuf};
-    uint8_t* masks[2] = {mask, mbuf};
-    const int64_t work = n * ch;
-    for (int p = 0; p < passes; ++p) {
-      int src = p & 1, dst = src ^ 1;
-      if (kind == SHB_DILATE_U8)
-        k_dilate<uint8_t><<<grid_for(work), kThreads, 0, st>>>((const uint8_t*)bufs[src], masks[src],
-                                                               (uint8_t*)bufs[dst], masks[dst], width, height, ch,
-                                                               changed, p);
-      else
-        k_dilate<float><<<grid_for(work), kThreads, 0, st>>>((const float*)bufs[src], masks[src], (float*)bufs[dst],
-                                                             masks[dst], width, height, ch, changed, p);
-      count_launch(ctx);
-    }
-    if (passes & 1) {
-      SHB_CUDA(cudaMemcpyAsync(pixels, bufs[1], pbytes, cudaMemcpyDeviceToDevice, st));
-      SHB_CUDA(cudaMemcpyAsync(mask, masks[1], (size_t)n, cudaMemcpyDeviceToDevice, st));
-    }
-    SHB_CUDA(cudaGetLastError());
-    return SHB_OK;
+    // the labels take two bytes a texel, no more than `need`
+    return dilate_passes(ctx, kind, width, height, pixels, mask, passes,
+                         reinterpret_cast<uint16_t*>(base + kNoAllocFlagBytes), reinterpret_cast<int*>(base));
   });
 }
