@@ -1,10 +1,14 @@
 // shb_capi.cu - the extern "C" boundary (include/shb.h): contexts, scene
 // upload and validation, and dispatch of every entry point to its kernels.
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "shb_internal.h"
@@ -116,6 +120,7 @@ void ctx_retain(shb_context* c) { c->refs.fetch_add(1); }
 void ctx_release(shb_context* c) {
   if (c->refs.fetch_sub(1) != 1) return;
   ::shb::DeviceScope _shb_device_scope(c->device);
+  if (c->host_pinned) cudaFreeHost(c->host_pinned);
   if (c->own_stream) {
     cudaStreamSynchronize(c->own_stream);
     cudaStreamDestroy(c->own_stream);
@@ -326,6 +331,39 @@ void polar_rotation(const float Lf[9], float Rout[9]) {
     }
 }
 
+// Host memory for a call's copies to the device: the context's page-locked
+// buffer, kept between calls, up to kKeptStaging bytes (allocating and
+// freeing page-locked memory per call would cost more than it saves), plain
+// memory beyond.
+struct HostStaging {
+  static constexpr size_t kKeptStaging = size_t(64) << 20;
+  char* ptr = nullptr;
+  std::unique_ptr<char[]> own;
+  shb_status reserve(shb_context* c, size_t n) {
+    if (n > kKeptStaging) {
+      own.reset(new char[n]);
+      ptr = own.get();
+      return SHB_OK;
+    }
+    if (n > c->host_pinned_bytes) {
+      if (c->host_pinned) cudaFreeHost(c->host_pinned);
+      c->host_pinned = nullptr;
+      c->host_pinned_bytes = 0;
+      const size_t want = std::min(kKeptStaging, std::max<size_t>(2 * n, size_t(1) << 20));
+      if (cudaHostAlloc(&c->host_pinned, want, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->host_pinned = nullptr;
+        own.reset(new char[n]);
+        ptr = own.get();
+        return SHB_OK;
+      }
+      c->host_pinned_bytes = want;
+    }
+    ptr = static_cast<char*>(c->host_pinned);
+    return SHB_OK;
+  }
+};
+
 template <class T>
 static shb_status upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
   SHB_TRY(b.reserve(sizeof(T) * (v.empty() ? 1 : v.size())));
@@ -526,67 +564,90 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
     if (!ctx) return bad("NULL argument");
     SHB_ON_DEVICE(ctx->device);
     cudaStream_t st = ctx->stream;
-    std::vector<float> ov, on, tuv, luv, ot, lin, rot;
-    std::vector<uint32_t> vidx, tgeom, vgeom;
-    std::vector<DGeom> geoms;
+    // The geometry's arrays, concatenated in a staging buffer of the context
+    // (page-locked, so that its copies run at the link's rate and beside the
+    // host's next ones).
+    const size_t ng = d->geometry_count;
+    std::vector<DGeom> geoms(ng);
     bool raster_ready = true;
     std::string raster_error;
-    ov.reserve(3 * nv_total);
-    on.assign(3 * nv_total, 0.f);
-    tuv.assign(2 * nv_total, 0.f);
-    luv.assign(2 * nv_total, 0.f);
-    ot.assign(4 * nv_total, 0.f);
-    uint32_t vbase = 0, pbase = 0;
-    for (uint32_t g = 0; g < d->geometry_count; ++g) {
+    uint64_t vbase = 0, pbase = 0;
+    for (size_t g = 0; g < ng; ++g) {
       const shb_geometry_desc& gd = d->geometries[g];
-      if (gd.vertex_count && !gd.vertices) return bad("geometry " + std::to_string(g) + ": vertices is NULL");
-      if (gd.index_count && !gd.indices) return bad("geometry " + std::to_string(g) + ": indices is NULL");
+      const std::string where = "geometry " + std::to_string(g);
+      if (gd.vertex_count && !gd.vertices) return bad(where + ": vertices is NULL");
+      if (gd.index_count && !gd.indices) return bad(where + ": indices is NULL");
       if (gd.material_id < -1 || (gd.material_id >= 0 && (uint32_t)gd.material_id >= d->material_count))
-        return bad("geometry " + std::to_string(g) + ": material_id out of range");
-      uint32_t ntri = gd.index_count / 3;
-      for (uint32_t i = 0; i < ntri * 3; ++i)
-        if (gd.indices[i] >= gd.vertex_count) return bad("geometry " + std::to_string(g) + ": index out of range");
-      DGeom G;
+        return bad(where + ": material_id out of range");
+      const uint32_t ntri = gd.index_count / 3;
+      uint32_t top = 0;
+      for (uint32_t i = 0; i < ntri * 3; ++i) top = std::max(top, gd.indices[i]);
+      if (ntri && top >= gd.vertex_count) return bad(where + ": index out of range");
+      DGeom& G = geoms[g];
       std::memset(&G, 0, sizeof(G));
-      G.vbase = vbase;
-      G.prim_base = pbase;
+      G.vbase = (uint32_t)vbase;
+      G.prim_base = (uint32_t)pbase;
       G.tri_count = ntri;
       G.material_id = gd.material_id;
       G.flags = (gd.normals ? GEOM_HAS_NORMALS : 0u) | (gd.texture_uvs ? GEOM_HAS_TEXUV : 0u) |
                 (gd.tangents ? GEOM_HAS_TANGENTS : 0u) | (gd.lightmap_uvs ? GEOM_HAS_LMUV : 0u);
-      geoms.push_back(G);
       if (gd.vertex_count == 0 || !gd.normals || !gd.tangents || !gd.lightmap_uvs) {
         if (raster_ready)
-          raster_error = "geometry " + std::to_string(g) +
-                         " lacks vertices, normals, tangents or lightmap_uvs (RasterizeScene requires them)";
+          raster_error = where + " lacks vertices, normals, tangents or lightmap_uvs (RasterizeScene requires them)";
         raster_ready = false;
       }
-      for (uint32_t v = 0; v < gd.vertex_count; ++v) {
-        uint64_t k = vbase + v;
-        for (int a = 0; a < 3; ++a) ov.push_back(gd.vertices[3 * v + a]);
-        if (gd.normals)
-          for (int a = 0; a < 3; ++a) on[3 * k + a] = gd.normals[3 * v + a];
-        if (gd.texture_uvs)
-          for (int a = 0; a < 2; ++a) tuv[2 * k + a] = gd.texture_uvs[2 * v + a];
-        if (gd.lightmap_uvs)
-          for (int a = 0; a < 2; ++a) luv[2 * k + a] = gd.lightmap_uvs[2 * v + a];
-        if (gd.tangents)
-          for (int a = 0; a < 4; ++a) ot[4 * k + a] = gd.tangents[4 * v + a];
-        vgeom.push_back(g);
-      }
-      for (uint32_t t = 0; t < ntri; ++t) {
-        for (int k = 0; k < 3; ++k) vidx.push_back(vbase + gd.indices[3 * t + k]);
-        tgeom.push_back(g);
-      }
-      for (int i = 0; i < 12; ++i) lin.push_back(gd.transform[i]);
-      float L[9] = {gd.transform[0], gd.transform[1], gd.transform[2], gd.transform[4], gd.transform[5],
-                    gd.transform[6], gd.transform[8], gd.transform[9], gd.transform[10]};
-      float R[9];
-      polar_rotation(L, R);
-      for (int i = 0; i < 9; ++i) rot.push_back(R[i]);
       vbase += gd.vertex_count;
       pbase += ntri;
     }
+    float *ov, *on, *tuv, *luv, *ot, *lin, *rot;
+    uint32_t *vidx, *tgeom, *vgeom;
+    size_t staged = 0;
+    HostStaging staging;
+    for (int pass = 0; pass < 2; ++pass) {
+      staged = 0;
+      auto take = [&](auto*& p, size_t n) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(staging.ptr + staged);
+        staged += (sizeof(*p) * n + 63) & ~size_t(63);
+      };
+      take(ov, 3 * vbase);
+      take(on, 3 * vbase);
+      take(tuv, 2 * vbase);
+      take(luv, 2 * vbase);
+      take(ot, 4 * vbase);
+      take(vidx, 3 * pbase);
+      take(tgeom, pbase);
+      take(vgeom, vbase);
+      take(lin, 12 * ng);
+      take(rot, 9 * ng);
+      if (pass == 0) SHB_TRY(staging.reserve(ctx, staged));
+    }
+    auto fill = [](float* dst, const float* src, size_t n) {
+      if (src) std::memcpy(dst, src, sizeof(float) * n);
+      else std::memset(dst, 0, sizeof(float) * n);
+    };
+    std::atomic<size_t> next_geom{0};
+    auto fill_geometries = [&] {
+      for (size_t g; (g = next_geom.fetch_add(1)) < ng;) {
+        const shb_geometry_desc& gd = d->geometries[g];
+        const DGeom& G = geoms[g];
+        const size_t v0 = G.vbase, p0 = G.prim_base, nv = gd.vertex_count;
+        fill(ov + 3 * v0, gd.vertices, 3 * nv);
+        fill(on + 3 * v0, gd.normals, 3 * nv);
+        fill(tuv + 2 * v0, gd.texture_uvs, 2 * nv);
+        fill(luv + 2 * v0, gd.lightmap_uvs, 2 * nv);
+        fill(ot + 4 * v0, gd.tangents, 4 * nv);
+        std::fill(vgeom + v0, vgeom + v0 + nv, (uint32_t)g);
+        for (size_t i = 0; i < 3 * (size_t)G.tri_count; ++i) vidx[3 * p0 + i] = (uint32_t)v0 + gd.indices[i];
+        std::fill(tgeom + p0, tgeom + p0 + G.tri_count, (uint32_t)g);
+        std::memcpy(lin + 12 * g, gd.transform, sizeof(float) * 12);
+        const float L[9] = {gd.transform[0], gd.transform[1], gd.transform[2], gd.transform[4], gd.transform[5],
+                            gd.transform[6], gd.transform[8], gd.transform[9], gd.transform[10]};
+        polar_rotation(L, rot + 9 * g);
+      }
+    };
+    // one thread per 4 MB: fewer bytes are copied before a thread has started
+    run_host_threads((unsigned)std::min<size_t>({staged >> 22, ng, 8, std::thread::hardware_concurrency()}),
+                     fill_geometries);
     std::vector<DMat> mats;
     std::vector<uint8_t> pix;
     int has_alpha = 0;
@@ -652,8 +713,8 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
     std::unique_ptr<shb_scene> owner(new shb_scene());  // owned here until handed out
     shb_scene* s = owner.get();
     s->ctx = ctx;
-    s->vertex_count = vbase;
-    s->prim_count = pbase;
+    s->vertex_count = (uint32_t)vbase;
+    s->prim_count = (uint32_t)pbase;
     s->geom_count = d->geometry_count;
     s->mat_count = d->material_count;
     s->light_count = d->light_count;
@@ -688,20 +749,26 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
     auto chk = [&](shb_status x) {
       if (rc == SHB_OK) rc = x;
     };
-    chk(upload(s->obj_v, ov, st));
-    chk(upload(s->obj_n, on, st));
-    chk(upload(s->tex_uv, tuv, st));
-    chk(upload(s->lm_uv, luv, st));
-    chk(upload(s->obj_t, ot, st));
-    chk(upload(s->tri_vidx, vidx, st));
-    chk(upload(s->tri_geom, tgeom, st));
-    chk(upload(s->vgeom, vgeom, st));
+    auto put = [&](DevBuf& dst, const auto* src, size_t n) {
+      chk(dst.reserve(sizeof(*src) * (n ? n : 1)));
+      if (rc != SHB_OK || n == 0) return;
+      const cudaError_t e = cudaMemcpyAsync(dst.ptr, src, sizeof(*src) * n, cudaMemcpyHostToDevice, st);
+      if (e != cudaSuccess) chk(cuda_fail(e, "scene upload"));
+    };
+    put(s->obj_v, ov, 3 * vbase);
+    put(s->obj_n, on, 3 * vbase);
+    put(s->tex_uv, tuv, 2 * vbase);
+    put(s->lm_uv, luv, 2 * vbase);
+    put(s->obj_t, ot, 4 * vbase);
+    put(s->tri_vidx, vidx, 3 * pbase);
+    put(s->tri_geom, tgeom, pbase);
+    put(s->vgeom, vgeom, vbase);
+    put(s->lin, lin, 12 * ng);
+    put(s->rot, rot, 9 * ng);
     chk(upload(s->geoms, geoms, st));
     chk(upload(s->mats, mats, st));
     chk(upload(s->pixels, pix, st));
     chk(upload(s->lights, lights, st));
-    chk(upload(s->lin, lin, st));
-    chk(upload(s->rot, rot, st));
     if (rc == SHB_OK) chk(s->world_v.reserve(sizeof(float) * 3 * (vbase ? vbase : 1)));
     if (rc == SHB_OK) chk(s->world_n.reserve(sizeof(float) * 3 * (vbase ? vbase : 1)));
     if (rc == SHB_OK) chk(s->world_t.reserve(sizeof(float) * 4 * (vbase ? vbase : 1)));
@@ -712,7 +779,10 @@ shb_status shb_scene_upload(shb_context* ctx, const shb_scene_desc* d, shb_scene
       cudaError_t e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) rc = cuda_fail(e, "scene upload");
     }
-    if (rc != SHB_OK) return rc;
+    if (rc != SHB_OK) {
+      cudaStreamSynchronize(st);  // queued copies still read the staging buffer
+      return rc;
+    }
     ctx_retain(s->ctx);
     *out = owner.release();
     return SHB_OK;
