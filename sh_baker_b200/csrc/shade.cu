@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
       N = sp.nrm;
       dw = primary_dir(sp, B->seed, texel, sample);
       o = sp.pos + sp.nrm * 0.001f;
-      a.info[p] = make_uint4(b, texel, sample, 0u);
+      __stcs(a.info + p, make_uint4(b, texel, sample, 0u));
       if (BWD) {
         // dLoss/dL of this path: sh_out = (1/spp) sum 2pi L Y(dw) (k_resolve)
         g = a.dsh + (int64_t)texel * 27;
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
       }
       int slot = warp_push(a.cnt + CNT_SHADOW, ok);
       if (ok && slot_ok(a, slot, a.sh_cap)) {
-        a.sh.o[slot] = make_float4(P0.x, P0.y, P0.z, e.tfar);
+        __stcs(&a.sh.o[slot], make_float4(P0.x, P0.y, P0.z, e.tfar));
         if (BWD) {
           // Li = rad / (joint nls) projected along the unnormalised ray
           // direction (k_resolve); the selection pdf is held constant.
@@ -819,20 +819,21 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
             a.pk[(int64_t)n++ * a.sh_cap + slot] = make_float4(v.x, v.y, v.z, __uint_as_float((uint32_t)e.pmat));
           }
           a.pend[slot] = make_float4(__uint_as_float(n), 0.f, 0.f, 0.f);
-          a.sh.d[slot] = make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z, __uint_as_float((uint32_t)slot));
-          a.sh.c[slot] = make_float4(0.f, 0.f, 0.f, __uint_as_float(2u | (b << 2)));
+          __stcs(&a.sh.d[slot], make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z, __uint_as_float((uint32_t)slot)));
+          __stcs(&a.sh.c[slot], make_float4(0.f, 0.f, 0.f, __uint_as_float(2u | (b << 2))));
         } else {
-          a.sh.d[slot] = make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z, __uint_as_float((uint32_t)(base * a.NLS + j)));
-          a.sh.c[slot] = make_float4(__uint_as_float(sharers), __uint_as_float((uint32_t)a.NLS), 0.f,
-                                     __uint_as_float(1u | (b << 2)));
+          __stcs(&a.sh.d[slot], make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z,
+                                            __uint_as_float((uint32_t)(base * a.NLS + j))));
+          __stcs(&a.sh.c[slot], make_float4(__uint_as_float(sharers), __uint_as_float((uint32_t)a.NLS), 0.f,
+                                            __uint_as_float(1u | (b << 2))));
         }
       }
     }
     int slot = warp_push(a.cnt + CNT_EXT0, active);
     if (active && slot_ok(a, slot, a.ext_cap)) {
-      a.ext[0].o[slot] = make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)p));
-      a.ext[0].d[slot] = make_float4(dw.x, dw.y, dw.z, __uint_as_float(1u));
-      a.ext[0].beta[slot] = make_float4(1.f, 1.f, 1.f, 0.f);  // w: tangent count 0
+      __stcs(&a.ext[0].o[slot], make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)p)));
+      __stcs(&a.ext[0].d[slot], make_float4(dw.x, dw.y, dw.z, __uint_as_float(1u)));
+      __stcs(&a.ext[0].beta[slot], make_float4(1.f, 1.f, 1.f, 0.f));  // w: tangent count 0
     }
   }
   // shadow_rays counts the light queries, shared or not
@@ -908,9 +909,9 @@ __device__ __forceinline__ void nee_hit(const WaveArgs& a, const BakeItem* B, ui
           kind = 2u;
         }
       }
-      a.sh.o[slot] = make_float4(hit_pos.x, hit_pos.y, hit_pos.z, e.tfar);
-      a.sh.d[slot] = make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z, __uint_as_float(target));
-      a.sh.c[slot] = make_float4(c.x, c.y, c.z, __uint_as_float(kind | (b << 2)));
+      __stcs(&a.sh.o[slot], make_float4(hit_pos.x, hit_pos.y, hit_pos.z, e.tfar));
+      __stcs(&a.sh.d[slot], make_float4(e.ray_d.x, e.ray_d.y, e.ray_d.z, __uint_as_float(target)));
+      __stcs(&a.sh.c[slot], make_float4(c.x, c.y, c.z, __uint_as_float(kind | (b << 2))));
     }
   }
 }
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
     int mat_id = -1;
     DMat mat{};
     if (active) {
-      float4 qo = q.o[i], qd = q.d[i], qb = q.beta[i], h = a.hits[i];
+      const float4 qo = __ldcs(q.o + i), qd = __ldcs(q.d + i), qb = __ldcs(q.beta + i), h = __ldcs(a.hits + i);
       path = __float_as_uint(qo.w);
       vertex = __float_as_uint(qd.w);
       d = {qd.x, qd.y, qd.z};
@@ -1003,9 +1004,9 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
       if (tr && slot_ok(a, slot, a.ext_cap)) {
         f3 hp = pos + d * 0.001f;
         f3 bt = beta * (1.0f - alpha);
-        qn.o[slot] = make_float4(hp.x, hp.y, hp.z, __uint_as_float(path));
-        qn.d[slot] = make_float4(d.x, d.y, d.z, __uint_as_float(2u * vertex + 1u));
-        qn.beta[slot] = make_float4(bt.x, bt.y, bt.z, __uint_as_float(BWD ? ntan : 0u));
+        __stcs(&qn.o[slot], make_float4(hp.x, hp.y, hp.z, __uint_as_float(path)));
+        __stcs(&qn.d[slot], make_float4(d.x, d.y, d.z, __uint_as_float(2u * vertex + 1u)));
+        __stcs(&qn.beta[slot], make_float4(bt.x, bt.y, bt.z, __uint_as_float(BWD ? ntan : 0u)));
         if (BWD)
           for (uint32_t k = 0; k < ntan; ++k) {
             float4 t = a.tan[cur][(int64_t)k * a.ext_cap + i];
@@ -1048,11 +1049,11 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
       const int rs = warp_push(a.cnt + CNT_NEE, lit);
       if (lit && slot_ok(a, rs, a.ext_cap)) {
         const int64_t C = a.ext_cap;
-        a.nee_rec[rs] = make_float4(hit_pos.x, hit_pos.y, hit_pos.z, __uint_as_float(path));
-        a.nee_rec[C + rs] = make_float4(N.x, N.y, N.z, __uint_as_float(vertex));
-        a.nee_rec[2 * C + rs] = make_float4(d.x, d.y, d.z, alpha);
-        a.nee_rec[3 * C + rs] = make_float4(aop.x, aop.y, aop.z, beta.x);
-        a.nee_rec[4 * C + rs] = make_float4(beta.y, beta.z, 0.f, 0.f);
+        __stcs(a.nee_rec + rs, make_float4(hit_pos.x, hit_pos.y, hit_pos.z, __uint_as_float(path)));
+        __stcs(a.nee_rec + C + rs, make_float4(N.x, N.y, N.z, __uint_as_float(vertex)));
+        __stcs(a.nee_rec + 2 * C + rs, make_float4(d.x, d.y, d.z, alpha));
+        __stcs(a.nee_rec + 3 * C + rs, make_float4(aop.x, aop.y, aop.z, beta.x));
+        __stcs(a.nee_rec + 4 * C + rs, make_float4(beta.y, beta.z, 0.f, 0.f));
       }
     }
     // indirect (src/material.cpp:113-162, src/baker.cpp:131-148)
@@ -1106,9 +1107,9 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
           }
         }
       }
-      qn.o[slot] = make_float4(hit_pos.x, hit_pos.y, hit_pos.z, __uint_as_float(path));
-      qn.d[slot] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(2u * vertex));
-      qn.beta[slot] = make_float4(nb.x, nb.y, nb.z, __uint_as_float(nt));
+      __stcs(&qn.o[slot], make_float4(hit_pos.x, hit_pos.y, hit_pos.z, __uint_as_float(path)));
+      __stcs(&qn.d[slot], make_float4(nd.x, nd.y, nd.z, __uint_as_float(2u * vertex)));
+      __stcs(&qn.beta[slot], make_float4(nb.x, nb.y, nb.z, __uint_as_float(nt)));
     }
   }
   if (BWD) grad_flush(sgrad, a.n_params, a.grad);
@@ -1136,18 +1137,18 @@ __global__ void __launch_bounds__(kThreads, AREA == AREA_PAIRS ? kNeePairBlocks 
     uint32_t path = 0, vertex = 0, texel = 0, sample = 0, b = 0;
     const BakeItem* B = a.bakes;
     if (active) {
-      const float4 r0 = a.nee_rec[i], r1 = a.nee_rec[C + i], r2 = a.nee_rec[2 * C + i],
-                   r3 = a.nee_rec[3 * C + i];
+      const float4 r0 = __ldcs(a.nee_rec + i), r1 = __ldcs(a.nee_rec + C + i), r2 = __ldcs(a.nee_rec + 2 * C + i),
+                   r3 = __ldcs(a.nee_rec + 3 * C + i);
       hit_pos = {r0.x, r0.y, r0.z};
       path = __float_as_uint(r0.w);
       N = {r1.x, r1.y, r1.z};
       vertex = __float_as_uint(r1.w);
       d = {r2.x, r2.y, r2.z};
       aop = {r3.x, r3.y, r3.z};
-      const float4 r4 = a.nee_rec[4 * C + i];
+      const float4 r4 = __ldcs(a.nee_rec + 4 * C + i);
       alpha = r2.w;
       beta = {r3.w, r4.x, r4.y};
-      const PathInfo pi = a.info[path];
+      const PathInfo pi = __ldcs(a.info + path);
       b = pi.x;
       B = a.bakes + b;
       texel = pi.y;
@@ -1252,13 +1253,13 @@ __global__ void __launch_bounds__(kThreads) k_resolve(WaveArgs a) {
     for (uint32_t s = lane; s < t.spp; s += 32) {
       int64_t p = pbase + s;
       for (int j = 0; j < nls; ++j) {
-        float4 li = a.nee_li[p * a.NLS + j];
+        const float4 li = __ldcs(a.nee_li + p * a.NLS + j);
         if (li.x != 0.f || li.y != 0.f || li.z != 0.f) {
-          float4 nd = a.nee_dir[p * a.NLS + j];
+          const float4 nd = __ldcs(a.nee_dir + p * a.NLS + j);
           sh_accumulate(f3{li.x, li.y, li.z}, f3{nd.x, nd.y, nd.z}, acc);
         }
       }
-      float4 L = a.path_L[p];
+      const float4 L = __ldcs(a.path_L + p);
       f3 dw = primary_dir(sp, B->seed, texel, s + B->sample_offset);
       sh_accumulate(f3{L.x, L.y, L.z} * two_pi, dw, acc);
       env += L.w;

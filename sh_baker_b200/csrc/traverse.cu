@@ -580,15 +580,15 @@ __global__ void SHB_TRAV_BOUNDS k_extend(BvhView one, const BakeItem* __restrict
   fill_perm(perm);
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&stats->extend_rays, (unsigned long long)n);
   auto load = [&](int i, float4& o, float4& d, float& tnear, float& tfar) {
-    o = q.o[i];
-    d = q.d[i];
+    o = __ldcs(q.o + i);
+    d = __ldcs(q.d + i);
     tnear = 0.001f;
     tfar = INFINITY;
     return ONE ? one : bakes[info[__float_as_uint(o.w)].x].bvh;
   };
   consume<false, ONE>(coop[threadIdx.x / 32], perm, one, n, fetch, err, max_iters, load,
                       [&](int i, const Walk& w, const HitRec& rec, const float4* tris) {
-                        hits[i] = hit_record(w, rec, tris);
+                        __stcs(hits + i, hit_record(w, rec, tris));
                       });
 }
 
@@ -604,16 +604,16 @@ __global__ void SHB_SHADOW_BOUNDS k_shadow(BvhView one, const BakeItem* __restri
   fill_perm(perm);
   if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&stats->shadow_rays, (unsigned long long)n);
   auto load = [&](int i, float4& o, float4& d, float& tnear, float& tfar) {
-    o = q.o[i];
-    d = q.d[i];
+    o = __ldcs(q.o + i);
+    d = __ldcs(q.d + i);
     tnear = 0.001f;
     tfar = o.w;
     return ONE ? one : bakes[__float_as_uint(q.c[i].w) >> 2].bvh;
   };
   consume<true, ONE>(coop[threadIdx.x / 32], perm, one, n, fetch, err, max_iters, load,
                      [&](int i, const Walk& w, const HitRec&, const float4*) {
-    float4 c = q.c[i];
-    uint32_t target = __float_as_uint(q.d[i].w);
+    const float4 c = __ldcs(q.c + i);
+    uint32_t target = __float_as_uint(__ldcs(&q.d[i].w));
     const uint32_t kind = __float_as_uint(c.w) & 3u;
     if (kind == 0u) {
       if (!w.hit) {

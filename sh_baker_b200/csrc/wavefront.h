@@ -7,6 +7,15 @@ namespace shb {
 
 constexpr uint32_t kMissPrim = 0xFFFFFFFFu;
 
+// Queue entries, hit records, next-event records and path infos are a stream:
+// each is written once and read once or twice, a whole wave later (a wave's
+// queues are several times the L2).  They are loaded and stored with evict-first
+// hints (.cs), which leaves the L2 to the tree, the triangles and the
+// attributes: 2,412-triangle room of 1,024^2 texels 62.5 -> 61.9 ms, 263k
+// triangles 255.5 -> 254.9, alpha leaves 10.43 -> 10.37, 128^2 lightmap
+// 7.31 -> 7.20.  The hints of the traversal or of the shading kernels alone
+// gave half of it.
+//
 // Extend (closest-hit) queue entry, structure of arrays:
 //   o    = (origin.xyz, path index bits)
 //   d    = (direction.xyz, path-vertex id bits)
