@@ -119,6 +119,7 @@ __global__ void k_tri_bbox(RasterArgs a, int4* __restrict__ box, int64_t* __rest
     int max_y = min(a.H - 1, cvt_trunc(ceilf(max_v * (float)a.H)));
     int bw = max_x - min_x + 1, bh = max_y - min_y + 1;
     box[p] = make_int4(min_x, min_y, bw, bh);
+    if (p == 0) area[a.T] = 0;  // the scan's last element: all candidates
     area[p] = (bw > 0 && bh > 0) ? (int64_t)bw * (int64_t)bh : 0;
   }
 }
@@ -126,7 +127,8 @@ __global__ void k_tri_bbox(RasterArgs a, int4* __restrict__ box, int64_t* __rest
 // One thread per candidate (triangle, texel) pair of all bounding boxes; the
 // last writer in geometry-major triangle order wins (atomicMax of the order).
 __global__ void k_cover(RasterArgs a, const int4* __restrict__ box, const int64_t* __restrict__ offs,
-                        int64_t total, int* __restrict__ owner, uint8_t* __restrict__ hit) {
+                        int* __restrict__ owner, uint8_t* __restrict__ hit) {
+  const int64_t total = offs[a.T];
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < total;
        c += (int64_t)gridDim.x * blockDim.x) {
     // upper_bound over the exclusive offsets
@@ -236,9 +238,17 @@ __global__ void k_resolve_raster(RasterArgs a, const int* __restrict__ owner, co
   }
 }
 
-__global__ void k_fill_i32(int* p, int64_t n, int v) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = v;
+// Start values of the texels' owners and fallbacks (three arrays of n) and
+// of the triangles' hit flags, in one launch (three fills and two memsets before).
+__global__ void k_raster_init(int* owner, int64_t n, uint8_t* hit, uint32_t T) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    owner[i] = -1;
+    owner[n + i] = 0x7FFFFFFF;
+    owner[2 * n + i] = -1;
+    if (i < T) hit[i] = 0;
+  }
+  for (int64_t i = n + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T; i += (int64_t)gridDim.x * blockDim.x)
+    hit[i] = 0;
 }
 
 // --------------------------------------------------------------- masks ----
@@ -464,20 +474,16 @@ shb_status rasterize_device(shb_scene* s, int W, int H, shb_surface_point* d_out
   int* owner = c->scratch[1].as<int>();
   int* fb_pos = owner + n;
   int* fb_neg = owner + 2 * n;
-  k_fill_i32<<<grid_for(n), kThreads, 0, st>>>(owner, n, -1);
-  k_fill_i32<<<grid_for(n), kThreads, 0, st>>>(fb_pos, n, 0x7FFFFFFF);
-  k_fill_i32<<<grid_for(n), kThreads, 0, st>>>(fb_neg, n, -1);
-  count_launch(c, 3);
+  SHB_TRY(c->scratch[4].reserve(T ? T : 1));
+  uint8_t* hit = c->scratch[4].as<uint8_t>();
+  k_raster_init<<<grid_for(n), kThreads, 0, st>>>(owner, n, hit, T);
+  count_launch(c);
   if (T > 0) {
     SHB_TRY(c->scratch[2].reserve(sizeof(int4) * T));
     SHB_TRY(c->scratch[3].reserve(sizeof(int64_t) * (T + 1) * 2));
-    SHB_TRY(c->scratch[4].reserve(T));
     int4* box = c->scratch[2].as<int4>();
     int64_t* area = c->scratch[3].as<int64_t>();
     int64_t* offs = area + (T + 1);
-    uint8_t* hit = c->scratch[4].as<uint8_t>();
-    SHB_CUDA(cudaMemsetAsync(hit, 0, T, st));
-    SHB_CUDA(cudaMemsetAsync(area + T, 0, sizeof(int64_t), st));
     k_tri_bbox<<<grid_for(T), kThreads, 0, st>>>(a, box, area);
     count_launch(c);
     size_t tmp_bytes = 0;
@@ -485,13 +491,10 @@ shb_status rasterize_device(shb_scene* s, int W, int H, shb_surface_point* d_out
     SHB_TRY(c->scratch[5].reserve(tmp_bytes));
     SHB_CUDA(cub::DeviceScan::ExclusiveSum(c->scratch[5].ptr, tmp_bytes, area, offs, (int64_t)T + 1, st));
     count_launch(c, 2);
-    int64_t total = 0;
-    SHB_CUDA(cudaMemcpyAsync(&total, offs + T, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    SHB_CUDA(cudaStreamSynchronize(st));
-    if (total > 0) {
-      k_cover<<<grid_for(total), kThreads, 0, st>>>(a, box, offs, total, owner, hit);
-      count_launch(c);
-    }
+    // The candidates' number stays on the device, so that the host does not wait
+    // for the scan; the grid is for about one per texel and a few per triangle.
+    k_cover<<<grid_for(n + 4 * (int64_t)T), kThreads, 0, st>>>(a, box, offs, owner, hit);
+    count_launch(c);
     k_fallback<<<grid_for(T), kThreads, 0, st>>>(a, hit, owner, fb_pos, fb_neg);
     count_launch(c);
   }

@@ -553,6 +553,7 @@ struct WaveArgs {
   float4* nee_li;
   float4* nee_dir;
   int* cnt;
+  Counters64* c64;
   int ext_cap;  // capacity of each extend queue
   int sh_cap;   // capacity of the shadow queue
   // With several light samples or alpha branching a path gets more than one
@@ -690,9 +691,10 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
       const Tile t = a.tiles[find_tile<true>(a, p)];
       b = t.bake;
       B = a.bakes + b;
-      int64_t local = p - t.path_off;
-      uint32_t slot = t.t0 + (uint32_t)(local / t.spp);
-      sample = (uint32_t)(local % t.spp) + B->sample_offset;
+      const uint32_t local = (uint32_t)(p - t.path_off);  // a wave has below 2^31 paths
+      const uint32_t in_tile = local / t.spp;
+      const uint32_t slot = t.t0 + in_tile;
+      sample = local - in_tile * t.spp + B->sample_offset;
       texel = B->valid[slot];
       SP sp = load_sp(B->pts, texel);
       P0 = sp.pos;
@@ -802,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
         shared_rays += __popc(__ballot_sync(0xFFFFFFFFu, ok)) - __popc(__ballot_sync(0xFFFFFFFFu, first));
         ok = first;
       }
-      int slot = warp_push(a.cnt + CNT_SHADOW, ok);
+      int slot = warp_push(a.cnt + depth_cnt(0, DC_SHADOW), ok);
       if (ok && slot_ok(a, slot, a.sh_cap)) {
         __stcs(&a.sh.o[slot], make_float4(P0.x, P0.y, P0.z, e.tfar));
         if (BWD) {
@@ -829,7 +831,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
         }
       }
     }
-    int slot = warp_push(a.cnt + CNT_EXT0, active);
+    int slot = warp_push(a.cnt + depth_cnt(0, DC_EXT), active);
     if (active && slot_ok(a, slot, a.ext_cap)) {
       __stcs(&a.ext[0].o[slot], make_float4(o.x, o.y, o.z, __uint_as_float((uint32_t)p)));
       __stcs(&a.ext[0].d[slot], make_float4(dw.x, dw.y, dw.z, __uint_as_float(1u)));
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
   }
   // shadow_rays counts the light queries, shared or not
   if (!BWD && lane == 0 && shared_rays)
-    atomicAdd(&reinterpret_cast<Counters64*>(a.cnt + CNT_COUNT)->shadow_rays, (unsigned long long)shared_rays);
+    atomicAdd(&a.c64->shadow_rays, (unsigned long long)shared_rays);
 }
 
 // --------------------------------------------------------------- shade ---
@@ -875,7 +877,7 @@ __device__ __forceinline__ void nee_hit(const WaveArgs& a, const BakeItem* B, ui
         scale = alpha / (joint * (float)nls);
       }
     }
-    int slot = warp_push(a.cnt + CNT_SHADOW, ok);
+    int slot = warp_push(a.cnt + depth_cnt(depth, DC_SHADOW), ok);
     if (ok && slot_ok(a, slot, a.sh_cap)) {
       uint32_t target = path, kind = 0u;
       if (BWD) {
@@ -932,7 +934,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
   // forward inline next-event estimation: the staged light table
   const DLight* wave_lights =
       (BWD || SPLIT) ? nullptr : stage_lights(a.bakes, a.one_bake, reinterpret_cast<DLight*>(sgrad));
-  const int n = min(a.cnt[cur], a.ext_cap);
+  const int n = min(a.cnt[depth_cnt(depth, DC_EXT)], a.ext_cap);
   const int nxt = cur ^ 1;
   const int warps = gridDim.x * (blockDim.x >> 5);
   const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
     // transmission (src/baker.cpp:99-105)
     if (__any_sync(0xFFFFFFFFu, hit && B->sc.has_alpha)) {
       bool tr = hit && alpha < 1.0f && can_extend;
-      int slot = warp_push(a.cnt + nxt, tr);
+      int slot = warp_push(a.cnt + depth_cnt(depth + 1, DC_EXT), tr);
       if (tr && slot_ok(a, slot, a.ext_cap)) {
         f3 hp = pos + d * 0.001f;
         f3 bt = beta * (1.0f - alpha);
@@ -1046,7 +1048,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
     } else {
       // a vertex seen from behind has a zero BRDF: no light weighs anything
       const bool lit = opaque_hit && !(dot(N, wo) <= 0.0f);
-      const int rs = warp_push(a.cnt + CNT_NEE, lit);
+      const int rs = warp_push(a.cnt + depth_cnt(depth, DC_NEE), lit);
       if (lit && slot_ok(a, rs, a.ext_cap)) {
         const int64_t C = a.ext_cap;
         __stcs(a.nee_rec + rs, make_float4(hit_pos.x, hit_pos.y, hit_pos.z, __uint_as_float(path)));
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
         if (BWD && !zero) hscale = alpha * ((cos_term / pdf) / 3.14159265358979323846f);
       }
     }
-    int slot = warp_push(a.cnt + nxt, ext);
+    int slot = warp_push(a.cnt + depth_cnt(depth + 1, DC_EXT), ext);
     if (ext && slot_ok(a, slot, a.ext_cap)) {
       uint32_t nt = 0;
       if (BWD) {
@@ -1116,14 +1118,14 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : SPLIT ? kShad
 }
 
 // Next-event estimation of the forward bake over the dense record queue
-// k_shade filled (CNT_NEE): the same arithmetic as the inline call of the
+// k_shade filled (DC_NEE): the same arithmetic as the inline call of the
 // adjoint, with fewer live registers and every lane on an opaque hit.
 template <int AREA>
 __global__ void __launch_bounds__(kThreads, AREA == AREA_PAIRS ? kNeePairBlocks : kNeeBlocks)
     k_nee(WaveArgs a, int cur, int depth) {
   extern __shared__ float dyn_smem[];
   const DLight* wave_lights = stage_lights(a.bakes, a.one_bake, reinterpret_cast<DLight*>(dyn_smem));
-  const int n = min(a.cnt[CNT_NEE], a.ext_cap);
+  const int n = min(a.cnt[depth_cnt(depth, DC_NEE)], a.ext_cap);
   const int warps = gridDim.x * (blockDim.x >> 5);
   const int warp_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -1162,10 +1164,10 @@ __global__ void __launch_bounds__(kThreads, AREA == AREA_PAIRS ? kNeePairBlocks 
 
 // Adds the gradient packets of the visible shadow rays (BWD): count in
 // pend[slot].x, cleared by k_shadow for occluded rays.
-__global__ void __launch_bounds__(kThreads) k_apply(WaveArgs a) {
+__global__ void __launch_bounds__(kThreads) k_apply(WaveArgs a, int depth) {
   extern __shared__ float sgrad[];
   grad_zero(sgrad, a.n_params);
-  const int n = min(a.cnt[CNT_SHADOW], a.sh_cap);
+  const int n = min(a.cnt[depth_cnt(depth, DC_SHADOW)], a.sh_cap);
   const int stride = gridDim.x * blockDim.x;
   for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
     const int i = base + (threadIdx.x & 31);
@@ -1389,12 +1391,12 @@ shb_status find_occlusion_device(shb_scene* s, const shb_ray* d_rays, int64_t n,
   shb_context* c = s->ctx;
   if (n <= 0) return SHB_OK;
   SHB_TRY(c->scratch[9].reserve(sizeof(float4) * (size_t)n));
-  SHB_TRY(c->counters.reserve(sizeof(int) * CNT_COUNT + sizeof(Counters64)));
+  SHB_TRY(c->counters.reserve(sizeof(int) * kCounterInts));
   int* cnt = c->counters.as<int>();
-  SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_COUNT, c->stream));
+  SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_DEPTH0, c->stream));
   float4* hits = c->scratch[9].as<float4>();
-  launch_closest_rays(c->stream, traversal_grid(c->device, false), s->bvh(), d_rays, n, hits, cnt + CNT_FETCH_EXT,
-                      cnt + CNT_ERROR);
+  launch_closest_rays(c->stream, traversal_grid(c->device, false), s->bvh(), d_rays, n, hits,
+                      cnt + depth_cnt(0, DC_FETCH_EXT), cnt + CNT_ERROR);
   k_occ_attrs<<<grid_for(n), kThreads, 0, c->stream>>>(s->view(), d_rays, hits, n, d_hits);
   count_launch(c, 2);
   SHB_CUDA(cudaGetLastError());
@@ -1520,11 +1522,12 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
   }
   // outputs and valid-texel lists
   SHB_TRY(c->scratch[10].reserve(sizeof(uint32_t) * (size_t)(total_texels + nb)));
-  SHB_TRY(c->counters.reserve(sizeof(int) * CNT_COUNT + sizeof(Counters64) + sizeof(int) * (size_t)nb));
+  const size_t cnt_bytes = sizeof(int) * kCounterInts + sizeof(Counters64) + sizeof(int) * (size_t)nb;
+  SHB_TRY(c->counters.reserve(cnt_bytes));
   int* cnt = c->counters.as<int>();
-  Counters64* c64 = reinterpret_cast<Counters64*>(cnt + CNT_COUNT);
+  Counters64* c64 = reinterpret_cast<Counters64*>(cnt + kCounterInts);
   int* nsel = reinterpret_cast<int*>(c64 + 1);
-  SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_COUNT + sizeof(Counters64) + sizeof(int) * (size_t)nb, st));
+  SHB_CUDA(cudaMemsetAsync(cnt, 0, cnt_bytes, st));
   std::vector<BakeItem> items(nb);
   uint32_t* valid_all = c->scratch[10].as<uint32_t>();
   int64_t voff = 0;
@@ -1628,6 +1631,7 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
   a.nee_dir = a.nee_li + std::max<int64_t>(Pmax, 1) * NLS;
   a.info = c->scratch[18].as<PathInfo>();
   a.cnt = cnt;
+  a.c64 = c64;
   a.ext_cap = (int)ext_cap;
   a.sh_cap = (int)sh_cap;
   a.det = det ? 1 : 0;
@@ -1709,7 +1713,8 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
     // traversal of a one-bake wave skips the per-ray bake lookup
     const int only = w.bake >= 0 ? w.bake : (nb == 1 ? 0 : -1);
     const BvhView* one = only >= 0 ? &items[only].bvh : nullptr;
-    cudaMemsetAsync(cnt, 0, sizeof(int) * (CNT_FETCH_SHADOW + 1), st);
+    if (&w != &waves.front())  // (the first wave's are clear)
+      cudaMemsetAsync(cnt + CNT_DEPTH0, 0, sizeof(int) * DC_COUNT * (size_t)(w.max_bounces + 2), st);
     Pair pg = stamp(2);
     a.one_bake = w.bake;
     by_area(w.area, [&](auto A) {
@@ -1719,15 +1724,12 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
     close_stamp(pg);
     launches++;
     for (int k = 0; k <= w.max_bounces; ++k) {
-      int cur = k & 1, nxt = cur ^ 1;
-      cudaMemsetAsync(cnt + nxt, 0, sizeof(int), st);
-      cudaMemsetAsync(cnt + CNT_FETCH_EXT, 0, sizeof(int) * 2, st);
+      const int cur = k & 1;
       Pair pe = stamp(0);
-      launch_extend(st, tgrid, one, d_items, a.info, a.ext[cur], cnt + cur, a.ext_cap, a.hits, cnt + CNT_FETCH_EXT,
-                    cnt + CNT_ERROR, c64, prm.max_iters);
+      launch_extend(st, tgrid, one, d_items, a.info, a.ext[cur], cnt + depth_cnt(k, DC_EXT), a.ext_cap, a.hits,
+                    cnt + depth_cnt(k, DC_FETCH_EXT), cnt + CNT_ERROR, c64, prm.max_iters);
       close_stamp(pe);
       Pair pd = stamp(2);
-      if (split_nee) cudaMemsetAsync(cnt + CNT_NEE, 0, sizeof(int), st);
       by_area(w.area, [&](auto A) {
         if (bwd) {
           k_shade<true, false, A.value><<<sgrid, kThreads, gsmem, st>>>(a, cur, k);
@@ -1741,14 +1743,13 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
       if (split_nee) launches++;
       close_stamp(pd);
       Pair ps = stamp(1);
-      launch_shadow(st, tgrid_sh, one, d_items, a.sh, cnt + CNT_SHADOW, a.sh_cap, a.path_L, a.nee_li, a.pend,
-                    cnt + CNT_FETCH_SHADOW, cnt + CNT_ERROR, c64, prm.max_iters);
+      launch_shadow(st, tgrid_sh, one, d_items, a.sh, cnt + depth_cnt(k, DC_SHADOW), a.sh_cap, a.path_L, a.nee_li,
+                    a.pend, cnt + depth_cnt(k, DC_FETCH_SHADOW), cnt + CNT_ERROR, c64, prm.max_iters);
       close_stamp(ps);
       if (bwd) {
-        k_apply<<<sgrid, kThreads, gsmem, st>>>(a);
+        k_apply<<<sgrid, kThreads, gsmem, st>>>(a, k);
         launches++;
       }
-      cudaMemsetAsync(cnt + CNT_SHADOW, 0, sizeof(int), st);
       launches += 3;
       if (det) {
         k_commit<<<grid_for(w.P), kThreads, 0, st>>>(a, k);

@@ -824,8 +824,9 @@ shb_status shb_scene_bvh_info(const shb_scene* s, uint32_t* wide_nodes, uint32_t
 namespace {
 
 // Rasterises into g (its storage grows as needed), optionally downloading
-// the points to host_out, and waits for the stream.
-shb_status rasterize_into(shb_scene* s, const shb_raster_config* cfg, shb_gbuffer* g, shb_surface_point* host_out) {
+// the points to host_out, and waits for the stream if asked.
+shb_status rasterize_into(shb_scene* s, const shb_raster_config* cfg, shb_gbuffer* g, shb_surface_point* host_out,
+                          bool wait) {
   if (!s->raster_ready) return bad(s->raster_error);
   if (cfg->width <= 0 || cfg->height <= 0 || cfg->supersample_scale <= 0)
     return bad("raster width, height and supersample_scale must be positive");
@@ -840,7 +841,7 @@ shb_status rasterize_into(shb_scene* s, const shb_raster_config* cfg, shb_gbuffe
   if (host_out)
     SHB_CUDA(cudaMemcpyAsync(host_out, g->points.ptr, sizeof(shb_surface_point) * (size_t)(W * H),
                              cudaMemcpyDeviceToHost, s->ctx->stream));
-  cudaError_t e = cudaStreamSynchronize(s->ctx->stream);
+  const cudaError_t e = wait ? cudaStreamSynchronize(s->ctx->stream) : cudaSuccess;
   if (e != cudaSuccess) return cuda_fail(e, "rasterize");
   return SHB_OK;
 }
@@ -854,7 +855,7 @@ shb_status shb_rasterize(shb_scene* s, const shb_raster_config* cfg, shb_surface
     if (out_gbuffer) *out_gbuffer = nullptr;
     std::unique_ptr<shb_gbuffer> owner(new shb_gbuffer());  // owned here until handed out
     shb_gbuffer* g = owner.get();
-    shb_status rc = rasterize_into(s, cfg, g, host_out);
+    shb_status rc = rasterize_into(s, cfg, g, host_out, true);
     if (rc != SHB_OK || !out_gbuffer) return rc;
     ctx_retain(g->ctx);
     *out_gbuffer = owner.release();
@@ -1220,7 +1221,7 @@ shb_status shb_bake_pipeline(shb_scene* s, const shb_pipeline_config* cfg, float
     shb_raster_config rc{cfg->width, cfg->height, ss};
     if (!c->pipe_gbuf) c->pipe_gbuf = new shb_gbuffer();
     shb_gbuffer* g = c->pipe_gbuf;
-    SHB_TRY(rasterize_into(s, &rc, g, nullptr));
+    SHB_TRY(rasterize_into(s, &rc, g, nullptr, false));
     const size_t W = (size_t)cfg->width * ss, H = (size_t)cfg->height * ss;
     const size_t n_hi = W * H, n_lo = (size_t)cfg->width * cfg->height;
     // device buffers: hi-res SH + env, hi-res mask, lo-res SH + env + mask

@@ -20,6 +20,8 @@
 // The watertight triangle test (Woop, Benthin, Wald 2013) uses explicit
 // round-to-nearest intrinsics so it rounds exactly like the CPU restatement
 // even though this file is compiled with FMA contraction for the box tests.
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 
 #include "f32x2.cuh"
@@ -658,13 +660,20 @@ __global__ void SHB_TRAV_BOUNDS k_closest_rays(BvhView bvh, const shb_ray* __res
 
 }  // namespace
 
+// Blocks that fill the device (asked of the runtime once per device: a query
+// takes longer than a launch).
 int traversal_grid(int device, bool shadow) {
+  static std::atomic<int> known[64][2];
+  if (device >= 0 && device < 64) {
+    const int g = known[device][shadow].load(std::memory_order_relaxed);
+    if (g > 0) return g;
+  }
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (shadow) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_shadow<true>, kTravThreads, 0);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_extend<true>, kTravThreads, 0);
-  if (per_sm < 1) per_sm = 1;
-  if (sms < 1) sms = 1;
+  if (per_sm < 1 || sms < 1) return std::max(per_sm, 1) * std::max(sms, 1);
+  if (device >= 0 && device < 64) known[device][shadow].store(sms * per_sm, std::memory_order_relaxed);
   return sms * per_sm;
 }
 

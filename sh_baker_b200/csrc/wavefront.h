@@ -40,17 +40,23 @@ struct ShadowQueue {
   float4* c;
 };
 
-// Device counters of one bake.
-enum CounterSlot {
-  CNT_EXT0 = 0,
-  CNT_EXT1 = 1,
-  CNT_SHADOW = 2,
-  CNT_FETCH_EXT = 3,
-  CNT_FETCH_SHADOW = 4,
-  CNT_ERROR = 5,
-  CNT_NEE = 6,  // next-event records of the current depth (forward bake)
-  CNT_COUNT = 8
+// Device counters of one bake: the error flags, then a set per depth of the
+// wave, so that one memset clears them all before the wave's first kernel.
+// (Four memsets a depth were half of a small bake's submissions: the 64^2
+// lightmap of a quad took 567 us with them and with the raster's host wait and
+// five fills, 500 us without.)
+enum CounterSlot { CNT_ERROR = 0, CNT_DEPTH0 = 8 };
+enum DepthSlot {
+  DC_EXT = 0,  // rays of the depth's extend queue
+  DC_SHADOW = 1,
+  DC_FETCH_EXT = 2,
+  DC_FETCH_SHADOW = 3,
+  DC_NEE = 4,  // next-event records (forward bake)
+  DC_COUNT = 8
 };
+constexpr int kMaxBounces = 30;  // bake configs have at most this many
+constexpr int kCounterInts = CNT_DEPTH0 + DC_COUNT * (kMaxBounces + 2);
+__host__ __device__ constexpr int depth_cnt(int depth, int slot) { return CNT_DEPTH0 + DC_COUNT * depth + slot; }
 enum ErrorBits : int { ERR_STACK = 1, ERR_QUEUE = 2, ERR_ITER = 4 };
 
 struct Counters64 {
