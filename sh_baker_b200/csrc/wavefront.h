@@ -45,17 +45,20 @@ struct ShadowQueue {
 // (Four memsets a depth were half of a small bake's submissions: the 64^2
 // lightmap of a quad took 567 us with them and with the raster's host wait and
 // five fills, 500 us without.)
-enum CounterSlot { CNT_ERROR = 0, CNT_DEPTH0 = 8 };
+enum CounterSlot { CNT_ERROR = 0, CNT_DEPTH0 = 9 };  // odd: see DC_NEE
 enum DepthSlot {
   DC_EXT = 0,  // rays of the depth's extend queue
   DC_SHADOW = 1,
   DC_FETCH_EXT = 2,
   DC_FETCH_SHADOW = 3,
-  DC_NEE = 4,  // next-event records (forward bake)
+  // next-event records (forward bake); with the next depth's DC_EXT, the int
+  // after it, one aligned 64-bit word
+  DC_NEE = 7,
   DC_COUNT = 8
 };
 constexpr int kMaxBounces = 30;  // bake configs have at most this many
-constexpr int kCounterInts = CNT_DEPTH0 + DC_COUNT * (kMaxBounces + 2);
+constexpr int kCounterInts = CNT_DEPTH0 + DC_COUNT * (kMaxBounces + 2) + 1;  // even
+static_assert((CNT_DEPTH0 + DC_NEE) % 2 == 0 && kCounterInts % 2 == 0 && DC_NEE + 1 == DC_COUNT && DC_EXT == 0, "");
 __host__ __device__ constexpr int depth_cnt(int depth, int slot) { return CNT_DEPTH0 + DC_COUNT * depth + slot; }
 enum ErrorBits : int { ERR_STACK = 1, ERR_QUEUE = 2, ERR_ITER = 4 };
 
