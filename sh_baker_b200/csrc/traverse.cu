@@ -63,6 +63,14 @@ constexpr int kTravThreads = 128;
 #define SHB_REFILL_MIN 10
 #endif
 constexpr int kRefillMin = SHB_REFILL_MIN;
+// Any hit: a warp fetches this many entries at once and hands them out from
+// shared memory.  Its walks are short, so the refills' adds to the one counter
+// queued up, most where a launch is short: batch of rooms 7.80 -> 7.19 ms, 128^2
+// lightmap of a room 7.03 -> 6.67; any hit of the 512^2 room 16.66 -> 16.55 and
+// of 263k triangles 56.4 -> 56.2.  Closest hit gains nothing there and is
+// slower with such a pool, 28.3 -> 29.4 and 83.0 -> 86.1: its walks are longer
+// and its registers and shared memory full.
+constexpr int kAnyChunk = 64;
 // 1: the warp-cooperative triangle phase; 0: each lane tests its own
 // triangles in a loop.
 #ifndef SHB_TRI_COOP
@@ -400,6 +408,7 @@ struct CoopWarp : CoopRays {
 };
 template <>
 struct CoopWarp<true> : CoopRays {
+  int2 pool;  // queue entries fetched and not yet taken (first, number)
   __device__ __forceinline__ void put(int, float, float, float, float) {}
   __device__ __forceinline__ void replay(Walk&, int, int) {}
   __device__ __forceinline__ HitRec rec(int) const { return HitRec(); }
@@ -504,8 +513,8 @@ __device__ __forceinline__ void fill_perm(PermTable& t) {
 // Persistent queue consumer: lanes refill from the queue as their rays end.
 // `load(i, o, d, tnear, tfar)` reads ray i and gives its bake's BVH.
 template <bool SHADOW, bool ONE, class Load, class Fin>
-__device__ __forceinline__ void consume(CoopWarp<SHADOW>& s, const PermTable& perm, const BvhView& one, int n, int* fetch,
-                                        int* err, uint32_t max_iters, Load&& load, Fin&& finish) {
+__device__ __forceinline__ void consume(CoopWarp<SHADOW>& s, const PermTable& perm, const BvhView& one, int n,
+                                        int* fetch, int* err, uint32_t max_iters, Load&& load, Fin&& finish) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint2 stack[kStack];
@@ -517,20 +526,40 @@ __device__ __forceinline__ void consume(CoopWarp<SHADOW>& s, const PermTable& pe
   int ray = -1;       // queue entry in flight
   int ended = -1;     // entry whose ray has ended but is not yet finished
   bool exhausted = false;
+  if constexpr (SHADOW) {
+    if (lane == 0) s.pool = make_int2(0, 0);
+    __syncwarp();
+  }
   while (true) {
     bool need = ray < 0 && !exhausted;
     unsigned needm = __ballot_sync(0xFFFFFFFFu, need);
     if (kRefillMin > 1 && __popc(needm) < kRefillMin && __any_sync(0xFFFFFFFFu, ray >= 0)) needm = 0;
     if (needm) {
-      int leader = __ffs(needm) - 1;
+      const int leader = SHADOW ? 0 : __ffs(needm) - 1;
       int base = 0;
-      if (lane == leader) base = atomicAdd(fetch, __popc(needm));
+      int2 pool;
+      if constexpr (SHADOW) {
+        pool = s.pool;
+        if (lane == 0 && __popc(needm) > pool.y) base = atomicAdd(fetch, kAnyChunk);
+      } else {
+        if (lane == leader) base = atomicAdd(fetch, __popc(needm));
+      }
       // the rays that ended since the last refill, together
       if (ended >= 0) finish(ended, w, s.rec(lane), (ONE ? one : own).tris);
       ended = -1;
       base = __shfl_sync(0xFFFFFFFFu, base, leader);
+      if constexpr (SHADOW) {
+        const int k = __popc(needm);
+        __syncwarp();  // every lane has read the pool
+        if (lane == 0)
+          s.pool = k > pool.y ? make_int2(base + k - pool.y, kAnyChunk + pool.y - k)
+                              : make_int2(pool.x + k, pool.y - k);
+        __syncwarp();
+      }
       if (need) {
-        int r = base + __popc(needm & lt);
+        int r = __popc(needm & lt);
+        if constexpr (SHADOW) r = r < pool.y ? pool.x + r : base + (r - pool.y);
+        else r += base;
         if (r < n) {
           ray = r;
           float4 o, d;

@@ -35,6 +35,21 @@ def test_waves_of_different_depths(gpu_ctx, depths, use_graph):
             assert env.cpu().numpy().tobytes() == renv.tobytes()
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 63, 64, 65, 129])
+def test_short_queues(gpu_ctx, n):
+    # about one light query per texel and per hit: queues around the entries
+    # that a warp fetches at once
+    sc = scenes.procedural_room(seed=12, n_boxes=6, res=16, n_point_lights=2)
+    rc = api.RasterConfig(n, 1, 1)
+    pts = api.RasterizeScene(sc, rc, ctx=gpu_ctx)
+    got = api.BakeSHLightMap(sc, pts, rc, api.BakeConfig(samples=1, bounces=1, seed=8), ctx=gpu_ctx)
+    ref = O.OracleScene(sc).bake(pts.reshape(-1), n, 1, 1, samples=1, bounces=1, seed=8)
+    g, r = got.sh_texture.reshape(n, 27), ref["sh"].reshape(n, 27)
+    off = ~np.isclose(g, r, rtol=2e-4, atol=2e-5 * max(1.0, float(np.abs(r).max()))).all(1)
+    assert off.sum() <= max(1, n // 50)  # paths that graze an edge
+    assert (got.environment_visibility_texture.reshape(-1) != ref["env"].reshape(-1)).sum() <= max(1, n // 50)
+
+
 @pytest.mark.parametrize("w,h,ss", [(1, 1, 1), (3, 5, 1), (7, 2, 3), (16, 16, 1)])
 def test_more_triangles_than_texels(gpu_ctx, w, h, ss):
     rng = np.random.default_rng(w)
