@@ -189,7 +189,7 @@ typedef struct shb_bake_stats {
   uint64_t texel_samples;  /* valid texels x samples                      */
   uint64_t valid_texels;
   uint64_t extend_rays;    /* closest-hit rays traced                     */
-  uint64_t shadow_rays;    /* any-hit rays traced                         */
+  uint64_t shadow_rays;    /* light queries (samples may share a ray)     */
   uint64_t kernel_launches;
   uint32_t error_flags;    /* device-side bounded-failure flags (0 = ok)  */
   uint32_t waves;
