@@ -560,7 +560,7 @@ __device__ __forceinline__ void consume(CoopWarp<SHADOW>& s, const PermTable& pe
         int r = __popc(needm & lt);
         if constexpr (SHADOW) r = r < pool.y ? pool.x + r : base + (r - pool.y);
         else r += base;
-        if (r < n) {
+        if (SHADOW ? (uint32_t)r < (uint32_t)n : r < n) {  // (the counter may pass 2^31 by the last fetches)
           ray = r;
           float4 o, d;
           float tnear, tfar;
