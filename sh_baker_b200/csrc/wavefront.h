@@ -19,7 +19,8 @@ constexpr uint32_t kMissPrim = 0xFFFFFFFFu;
 // Extend (closest-hit) queue entry, structure of arrays:
 //   o    = (origin.xyz, path index bits)
 //   d    = (direction.xyz, path-vertex id bits)
-//   beta = (throughput.xyz, unused)
+//   beta = (throughput.xyz, tangent count of the adjoint); not stored for a
+//          path's first ray, whose throughput is 1
 struct ExtQueue {
   float4* o;
   float4* d;
