@@ -480,9 +480,12 @@ __device__ __forceinline__ void load_ray(TravRay& r, float4 o, float4 d) {
   r.ox = o.x;
   r.oy = o.y;
   r.oz = o.z;
-  r.dx = d.x;
-  r.dy = d.y;
-  r.dz = d.z;
+  // (+ 0 turns -0 into +0: prepare takes the octant from < 0 and the
+  // reciprocal from the sign bit, and a ray along (-0, 1, -0), as a light of
+  // direction (0, -1, 0) sends it, missed every box)
+  r.dx = d.x + 0.0f;
+  r.dy = d.y + 0.0f;
+  r.dz = d.z + 0.0f;
   prepare(r);
 }
 
