@@ -778,6 +778,11 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
         } else {
           // inactive lanes evaluate too (their weights are dropped below)
           k = next_weights<AREA, false>(BL->sc, ll, i, P0, N, nm, ev, true, zero3, wa, wb);
+          // The lanes sample points of their own, and one that cannot take
+          // the pair (a distance out of pair_weights' range) has light i
+          // alone.  The step is the warp's, so that all lanes meet the
+          // shuffle above: the others weigh light i + 1 again.
+          k = __all_sync(0xFFFFFFFFu, !active || k == 2u) ? 2u : 1u;
         }
         sum += wa;
         cum[i] = sum;
