@@ -299,11 +299,12 @@ __device__ LightEval eval_light(const SceneView& sc, const DLight* lights, uint3
 // stream's uniform `u` against the running float sum; zero-weight lights
 // are never picked).
 // The running sums of up to kWeightCache lights are kept from the summing
-// pass in `cum`; they never fall unless a light is negative
-// (SceneView::negative_lights), so the pick is a binary search over them.
-// Otherwise, and when no sum exceeds the target (a uniform next to 1, an
-// overflow), the weights are evaluated again in order.  Either way the
-// picked light is evaluated once, after the search, for all lanes at once.
+// pass in `cum`.  They never fall unless a light is negative
+// (SceneView::negative_lights), so the pick is a binary search over them;
+// sums that may fall are searched in order.  The weights are evaluated again
+// only for longer tables and when no sum exceeds the target (a uniform next
+// to 1, an overflow).  In each case the picked light is evaluated once, after
+// the search, for all lanes at once.
 // `lights` is the bake's light table in global memory or the block's copy
 // of it in shared memory.
 constexpr uint32_t kWeightCache = 32;
@@ -318,11 +319,15 @@ __device__ __forceinline__ bool pick_light(const SceneView& sc, const DLight* li
                                            bool wo_back, f3 aop, float sum, float u, const float* cum, LightEval& out) {
   const float target = u * sum;
   int pick = -1;
-  if (sc.light_count <= kWeightCache && !sc.negative_lights) {
+  if (sc.light_count <= kWeightCache) {
     uint32_t pos = 0;
+    if (!sc.negative_lights) {
 #pragma unroll
-    for (uint32_t step = kWeightCache / 2; step > 0; step >>= 1)
-      if (pos + step < sc.light_count && !(target < cum[pos + step - 1])) pos += step;
+      for (uint32_t step = kWeightCache / 2; step > 0; step >>= 1)
+        if (pos + step < sc.light_count && !(target < cum[pos + step - 1])) pos += step;
+    } else {
+      while (pos + 1 < sc.light_count && !(target < cum[pos])) ++pos;
+    }
     if (target < cum[pos]) pick = (int)pos;
   }
   if (pick < 0) {
