@@ -369,8 +369,11 @@ __device__ __forceinline__ bool box_behind(const DLight& L, f3 P, f3 N, float nm
 // issue and by the latency of its dependent steps: k_nee on the 263k-triangle
 // atrium executes 28 % fewer instructions than with a light at a time
 // (shading of the 768^2 bake 141.0 -> 114.8 ms with the binary search of the
-// pick, the boxes and the register limits above).  False (nothing written) when a distance lies outside 2^-30 ..
-// 2^30, where a quotient could leave the normal range, or is NaN.
+// pick, the boxes and the register limits above).  False (nothing written)
+// when a distance is NaN or outside kPairNear .. kPairFar, where an emission's
+// quotient could leave the normal range.  (A direction's component below 2^-96
+// may still have a quotient that underflows and rounds differently; in the
+// cosine it is nothing beside the other two, unless they add up to exactly 0.)
 template <int AREA, bool HIT>
 __device__ __forceinline__ bool pair_weights(const SceneView& sc, const DLight& A, const DLight& B, f3 P, f3 N,
                                              Event& ev, bool wo_back, f3 aop, float& wa, float& wb) {
@@ -401,8 +404,7 @@ __device__ __forceinline__ bool pair_weights(const SceneView& sc, const DLight& 
   f32x2 lx = add2(tx, dup2(-P.x)), ly = add2(ty, dup2(-P.y)), lz = add2(tz, dup2(-P.z));
   const float2 dsq = unpack2(add2(mul2(lx, lx), add2(mul2(ly, ly), mul2(lz, lz))));
   const float da = sqrtf(dsq.x), db = sqrtf(dsq.y);
-  constexpr float lo = 0x1p-30f, hi = 0x1p30f;
-  if (!(da >= lo && da <= hi && db >= lo && db <= hi)) return false;
+  if (!(da >= kPairNear && da <= kPairFar && db >= kPairNear && db <= kPairFar)) return false;
   const f32x2 nd = pack2(-da, -db), rd = pack2(__frcp_rn(da), __frcp_rn(db));
   lx = div2(lx, nd, rd);
   ly = div2(ly, nd, rd);

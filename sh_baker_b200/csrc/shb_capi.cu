@@ -223,10 +223,8 @@ void light_consts(shb_scene* s) {
         if (sampled && known) L.pair = PAIR_AREA;
       }
     }
-    // pair_weights divides these by squared distances within 2^+-60: they
-    // must be 0 or keep the quotient and its residual in range
     for (float e : {L.er, L.eg, L.eb})
-      if (!(e == 0.f || (std::fabs(e) >= 0x1p-90f && std::fabs(e) <= 0x1p30f))) L.pair = PAIR_NONE;
+      if (!(e == 0.f || (std::fabs(e) >= kPairDim && std::fabs(e) <= kPairBright))) L.pair = PAIR_NONE;
     L.grey = L.er == L.eg && L.er == L.eb;
   }
   s->area_kind = s->area_light_count ? AREA_SINGLE : AREA_NONE;

@@ -202,6 +202,11 @@ struct DLight {
 // some whose weights are taken in pairs.
 enum : int { AREA_NONE = 0, AREA_SINGLE = 1, AREA_PAIRS = 2 };
 enum : int32_t { PAIR_NONE = 0, PAIR_POINT = 1, PAIR_AREA = 2 };
+// What lights weighed in pairs may be: their radiance before the distance (0
+// or between kPairDim and kPairBright per channel) and distances from kPairNear
+// to kPairFar.  Quotients by the squared distance then lie in 2^-120 .. 2^90
+// and their residuals above 2^-108, where div2 (f32x2.cuh) rounds correctly.
+constexpr float kPairDim = 0x1p-60f, kPairBright = 0x1p30f, kPairNear = 0x1p-30f, kPairFar = 0x1p30f;
 
 // Compressed 8-wide BVH node (80 bytes).  Children boxes are quantised on
 // a per-node power-of-two grid anchored at p; slot s holds the child whose
