@@ -115,6 +115,8 @@ def pack_scene(scene: Scene):
     n = len(scene.geometries)
     table = bytearray(_GEOMETRY.size * max(1, n))
     for i, g in enumerate(scene.geometries):
+        if g.vertices is None:
+            raise TypeError(f"geometry {i} has no vertices")
         v, nv = _rows(g.vertices, 3, keep)
         idx = g.indices
         if not (type(idx) is np.ndarray and idx.dtype == np.uint32 and idx.ndim == 1 and idx.flags.c_contiguous):
