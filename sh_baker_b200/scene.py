@@ -122,10 +122,13 @@ def pack_scene(scene: Scene):
         if not (type(idx) is np.ndarray and idx.dtype == np.uint32 and idx.ndim == 1 and idx.flags.c_contiguous):
             idx = np.ascontiguousarray(np.asarray(idx, dtype=np.uint32).reshape(-1))
         keep.append(idx)
+        mat = int(g.material_id)
+        if not -1 << 31 <= mat < 1 << 31:
+            mat = C.c_int32(mat).value  # its low 32 bits, as a ctypes field takes them
         _GEOMETRY.pack_into(table, i * _GEOMETRY.size, v, _rows(g.normals, 3, keep)[0],
                             _rows(g.texture_uvs, 2, keep)[0], _rows(g.lightmap_uvs, 2, keep)[0],
                             _rows(g.tangents, 4, keep)[0], nv,
-                            idx.__array_interface__["data"][0] if idx.size else 0, idx.size, int(g.material_id),
+                            idx.__array_interface__["data"][0] if idx.size else 0, idx.size, mat,
                             *np.asarray(g.transform, dtype=np.float32).reshape(3, 4).reshape(-1).tolist())
     geos = (A.GeometryDesc * max(1, n)).from_buffer(table)
     mats = (A.MaterialDesc * max(1, len(scene.materials)))()

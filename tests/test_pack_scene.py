@@ -1,5 +1,7 @@
 """pack_scene takes and refuses what setting the descriptor's fields one by
-one takes and refuses: a geometry without vertices is a TypeError."""
+one takes and refuses: a geometry without vertices is a TypeError, and a
+material id is the low 32 bits of whatever integer it is given as (an
+unsigned -1 among them)."""
 import numpy as np
 import pytest
 
@@ -12,6 +14,13 @@ def test_missing_vertices_are_refused():
     for indices in (np.zeros(0, np.uint32), np.arange(3, dtype=np.uint32)):
         with pytest.raises(TypeError):
             pack_scene(Scene([Geometry(vertices=None, indices=indices)], [], []))
+
+
+@pytest.mark.parametrize("given,packed", [(0, 0), (-1, -1), (np.uint32(0xFFFFFFFF), -1), (2 ** 32 + 3, 3),
+                                          (np.int64(7), 7), (2 ** 31, -2 ** 31)])
+def test_material_ids_wrap(given, packed):
+    desc, keep = pack_scene(Scene([Geometry(**TRI, material_id=given)], [Material()], []))
+    assert desc.geometries[0].material_id == packed and keep
 
 
 def test_forms_of_arrays():
