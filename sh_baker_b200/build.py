@@ -6,6 +6,7 @@ FMA contraction (their exact steps use explicit rounding intrinsics).
 """
 from __future__ import annotations
 
+import hashlib
 import os
 import subprocess
 import sys
@@ -33,6 +34,8 @@ SOURCES = {
     "atlas.cpp": [],
     "preview.cu": ["-fmad=false"],
 }
+# What the time of a batch's launches depends on; see kernel_id.
+KERNELS = ["shade.cu", "traverse.cu", "bvh_build.cu", "wavefront.h", "shb_internal.h", "shb_math.cuh", "f32x2.cuh"]
 HEADERS = ["shb_internal.h", "shb_math.cuh", "wavefront.h", "f32x2.cuh", "tspace.h"]
 
 
@@ -46,6 +49,15 @@ def _newer(out: Path, deps) -> bool:
         return True
     t = out.stat().st_mtime
     return any(Path(d).stat().st_mtime > t for d in deps)
+
+
+def kernel_id(defines=(), file_flags=None) -> str:
+    """Names the bake's kernels as they are built: their sources, flags and
+    defines.  The batch autotuner keeps its choices under it."""
+    h = hashlib.sha256(repr((ARCH, COMMON, SOURCES, tuple(defines), sorted((file_flags or {}).items()))).encode())
+    for f in KERNELS:
+        h.update((CSRC / f).read_bytes())
+    return "k" + h.hexdigest()[:12]
 
 
 def build(verbose: bool = False, force: bool = False, variant: str | None = None, defines=(),
@@ -66,8 +78,13 @@ def build(verbose: bool = False, force: bool = False, variant: str | None = None
         s = CSRC / src
         o = build_dir / (src + ".o")
         objs.append(o)
-        if force or _newer(o, [s, *headers, Path(__file__)]):
-            cmds.append([nvcc(), *ARCH, *COMMON, *flags, *file_flags.get(src, []), *dflags, "-c", str(s), "-o", str(o)])
+        deps, own = [s, *headers, Path(__file__)], []
+        if src == "batch.cu":
+            deps += [CSRC / k for k in KERNELS]
+            own = ["-DSHB_KERNEL_ID=" + kernel_id(defines, file_flags)]
+        if force or _newer(o, deps):
+            cmds.append([nvcc(), *ARCH, *COMMON, *flags, *file_flags.get(src, []), *dflags, *own, "-c", str(s), "-o",
+                         str(o)])
     if cmds:
         from concurrent.futures import ThreadPoolExecutor
 

@@ -17,8 +17,10 @@
 // Tuning is a coordinate descent over those four parameters, each candidate
 // timed with CUDA events on the whole batch (sample counts thinned evenly
 // when the batch holds more than 2^30 paths); the fastest per path is
-// appended as "<gpu>|v2|<class> wave tile grid share ms" to the tuning file so
-// later batches of the same class skip the search.
+// appended as "<gpu>|<kernels>|<class> wave tile grid share ms" to the tuning
+// file so later batches of the same class skip the search.  <kernels> names
+// the kernel sources and flags of the build (build.py kernel_id): a choice
+// timed with other kernels is not taken over.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -31,6 +33,12 @@
 #include <vector>
 
 #include "shb_internal.h"
+
+#ifndef SHB_KERNEL_ID
+#error "build.py defines SHB_KERNEL_ID"
+#endif
+#define SHB_STRING_(x) #x
+#define SHB_STRING(x) SHB_STRING_(x)
 
 namespace shb {
 namespace {
@@ -225,7 +233,7 @@ extern "C" shb_status shb_bake_batch(shb_context* ctx, const shb_batch_item* ite
     prm.tile_texels = int64_t(1) << 13;
     if (options && options->autotune) {
       const std::string file = tune_path(options->tune_cache);
-      const std::string key = device_name(ctx->device) + "|v2|" + shape_class(specs);
+      const std::string key = device_name(ctx->device) + "|" SHB_STRING(SHB_KERNEL_ID) "|" + shape_class(specs);
       if (!lookup(file, key, &prm)) {
         double cost = 0;
         BatchParams best;
