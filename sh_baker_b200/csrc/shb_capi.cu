@@ -332,8 +332,12 @@ void polar_rotation(const float Lf[9], float Rout[9]) {
 // buffer, kept between calls, at most kKeptStaging bytes (allocating and
 // freeing page-locked memory per call would cost more than it saves), or
 // plain memory where it cannot be had.
+// Locking a MiB takes about 0.6 ms, which a context's first upload waits for:
+// with up to 64 MiB, and twice what was asked, the first upload of 900,000
+// bare vertices took 44 ms and of 300,000 22 ms, with plain memory 33 and 16;
+// with this size 24 and 16.  Later uploads take the same with either.
 struct HostStaging {
-  static constexpr size_t kKeptStaging = size_t(64) << 20;
+  static constexpr size_t kKeptStaging = size_t(32) << 20;
   char* ptr = nullptr;
   std::unique_ptr<char[]> own;
   void reserve(shb_context* c, size_t n) {  // n <= kKeptStaging
@@ -341,7 +345,8 @@ struct HostStaging {
       if (c->host_pinned) cudaFreeHost(c->host_pinned);
       c->host_pinned = nullptr;
       c->host_pinned_bytes = 0;
-      const size_t want = std::min(kKeptStaging, std::max<size_t>(2 * n, size_t(1) << 20));
+      constexpr size_t kMiB = size_t(1) << 20;
+      const size_t want = std::min(kKeptStaging, (n + n / 8 + kMiB - 1) / kMiB * kMiB);
       if (cudaHostAlloc(&c->host_pinned, want, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         c->host_pinned = nullptr;
@@ -372,25 +377,27 @@ static shb_status upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
 // Copies a scene's geometry arrays, concatenated over the geometries, to the
 // device: through the context's staging buffer, so that the copies run at the
 // link's rate and beside the host's next ones.  What fits the buffer is laid
-// out in it whole; more goes through its two halves in turn.  (In plain memory
-// of its own such an upload waited for fresh pages: 1.2 M vertices with all
-// attributes in one geometry took 40 ms, now 5.4 ms; 9.6 M 345, now 40 ms.)
-// The caller waits for the stream before the next use of the buffer.
+// out in it whole and sent; more goes in pieces through its two halves in turn.
+// (In plain memory of its own such an upload waited for fresh pages: 1.2 M
+// vertices with all attributes in one geometry took 40 ms, now 5.6 ms; 9.6 M
+// 345, now 38 ms.)  The caller waits for the stream before the next use of the
+// buffer.
 static shb_status upload_geometry(shb_context* ctx, shb_scene* s, const shb_scene_desc* d,
                                   const std::vector<DGeom>& geoms, size_t nv, size_t nt) {
   cudaStream_t st = ctx->stream;
   const size_t ng = geoms.size();
-  enum Kind { VERTICES, NORMALS, TEX_UVS, LM_UVS, TANGENTS, VERTEX_GEOM, TRI_VIDX, TRI_GEOM, LINEAR, ROTATION, KINDS };
+  enum Kind { VERTICES, NORMALS, TEX_UVS, LM_UVS, TANGENTS, TRI_VIDX, TRI_GEOM, VERTEX_GEOM, LINEAR, ROTATION, KINDS };
   enum Per { VERTEX, TRIANGLE, GEOMETRY };
   struct Array {
     DevBuf* dst;
     Per per;
     size_t bytes;  // of one vertex, triangle or geometry
   };
-  const Array arrays[KINDS] = {{&s->obj_v, VERTEX, 12},   {&s->obj_n, VERTEX, 12}, {&s->tex_uv, VERTEX, 8},
-                               {&s->lm_uv, VERTEX, 8},    {&s->obj_t, VERTEX, 16}, {&s->vgeom, VERTEX, 4},
-                               {&s->tri_vidx, TRIANGLE, 12}, {&s->tri_geom, TRIANGLE, 4},
-                               {&s->lin, GEOMETRY, 48},   {&s->rot, GEOMETRY, 36}};
+  const Array arrays[KINDS] = {{&s->obj_v, VERTEX, 12},      {&s->obj_n, VERTEX, 12},     {&s->tex_uv, VERTEX, 8},
+                               {&s->lm_uv, VERTEX, 8},       {&s->obj_t, VERTEX, 16},     {&s->tri_vidx, TRIANGLE, 12},
+                               {&s->tri_geom, TRIANGLE, 4},  {&s->vgeom, VERTEX, 4},      {&s->lin, GEOMETRY, 48},
+                               {&s->rot, GEOMETRY, 36}};
+  auto padded = [](size_t n) { return (n + 63) & ~size_t(63); };
   auto count = [&](Per per) { return per == VERTEX ? nv : (per == TRIANGLE ? nt : ng); };
   // Elements first .. first + n of geometry g's part of an array.
   auto fill = [&](Kind kind, size_t g, size_t first, size_t n, char* out) {
@@ -432,16 +439,19 @@ static shb_status upload_geometry(shb_context* ctx, shb_scene* s, const shb_scen
   size_t offset[KINDS], total = 0;
   for (int k = 0; k < KINDS; ++k) {
     offset[k] = total;
-    total += (arrays[k].bytes * count(arrays[k].per) + 63) & ~size_t(63);
+    total += padded(arrays[k].bytes * count(arrays[k].per));
     SHB_TRY(arrays[k].dst->reserve(arrays[k].bytes * std::max<size_t>(count(arrays[k].per), 1)));
   }
-  const size_t threads = std::min<size_t>(8, std::thread::hardware_concurrency());
+  // one thread per 4 MB: fewer bytes are copied before a thread has started
+  auto threads_for = [](size_t bytes, size_t jobs) {
+    return (unsigned)std::min<size_t>({bytes >> 22, jobs, 8, std::thread::hardware_concurrency()});
+  };
   HostStaging staging;
   staging.reserve(ctx, std::min(total, HostStaging::kKeptStaging));
   if (total <= HostStaging::kKeptStaging) {
+    // (geometry by geometry: array by array the atrium's upload took 6 % longer)
     std::atomic<size_t> next{0};
-    // one thread per 4 MB: fewer bytes are copied before a thread has started
-    run_host_threads((unsigned)std::min<size_t>({total >> 22, ng, threads}), [&] {
+    run_host_threads(threads_for(total, ng), [&] {
       for (size_t g; (g = next.fetch_add(1)) < ng;)
         for (int k = 0; k < KINDS; ++k) {
           const Array& a = arrays[k];
@@ -455,45 +465,77 @@ static shb_status upload_geometry(shb_context* ctx, shb_scene* s, const shb_scen
                                  cudaMemcpyHostToDevice, st));
     return SHB_OK;
   }
-  struct Done {  // the copy out of a half
+  struct Done {  // the copies out of a half
     cudaEvent_t e = nullptr;
     ~Done() {
       if (e) cudaEventDestroy(e);
     }
   } done[2];
   for (Done& h : done) SHB_CUDA(cudaEventCreateWithFlags(&h.e, cudaEventDisableTiming));
-  constexpr size_t kHalf = HostStaging::kKeptStaging / 2, kGrain = size_t(1) << 20;
+  constexpr size_t cap = HostStaging::kKeptStaging / 2;
+  struct Segment {  // elements first .. first + n of an array, at `at` in the piece
+    Kind kind;
+    size_t first, n, at;
+  };
+  std::vector<Segment> piece;
+  size_t used = 0;
   int half = 0;
-  for (int k = 0; k < KINDS; ++k) {
-    const Array& a = arrays[k];
-    const size_t all = count(a.per), piece = kHalf / a.bytes, grain = kGrain / a.bytes;
-    for (size_t p0 = 0; p0 < all; p0 += piece, half ^= 1) {
-      const size_t p1 = std::min(all, p0 + piece);
-      char* out = staging.ptr + half * kHalf;
-      SHB_CUDA(cudaEventSynchronize(done[half].e));  // (returns at once before the first record)
-      std::atomic<size_t> next{p0};
-      run_host_threads((unsigned)std::min<size_t>((p1 - p0) * a.bytes >> 22, threads), [&] {
-        for (size_t i; (i = next.fetch_add(grain)) < p1;) {
-          const size_t end = std::min(p1, i + grain);
-          size_t lo = 0, hi = ng;  // the last geometry that begins at or before i
-          while (hi - lo > 1) {
-            const size_t mid = (lo + hi) / 2;
-            if (first_of(a.per, mid) <= i) lo = mid;
-            else hi = mid;
-          }
-          for (size_t g = lo; i < end; ++g) {
-            const size_t in = i - first_of(a.per, g), n = std::min(end - i, count_of(a.per, g) - in);
-            if (n) fill((Kind)k, g, in, n, out + (i - p0) * a.bytes);
-            i += n;
-          }
+  auto fill_piece = [&](char* base) {
+    // a job is 256 KB or, where a rotation is computed for each, 8 geometries
+    auto per_job = [&](const Segment& g) {
+      return arrays[g.kind].per == GEOMETRY ? size_t(8) : (size_t(1) << 18) / arrays[g.kind].bytes;
+    };
+    auto jobs_of = [&](const Segment& g) { return (g.n + per_job(g) - 1) / per_job(g); };
+    size_t jobs = 0;
+    for (const Segment& g : piece) jobs += jobs_of(g);
+    std::atomic<size_t> next{0};
+    run_host_threads(threads_for(used, jobs), [&] {
+      for (size_t j; (j = next.fetch_add(1)) < jobs;) {
+        const Segment* sg = piece.data();
+        while (j >= jobs_of(*sg)) j -= jobs_of(*sg++);
+        const Array& a = arrays[sg->kind];
+        size_t i = sg->first + j * per_job(*sg);
+        const size_t end = std::min(sg->first + sg->n, i + per_job(*sg));
+        size_t lo = 0, hi = ng;  // the last geometry that begins at or before i
+        while (hi - lo > 1) {
+          const size_t mid = (lo + hi) / 2;
+          if (first_of(a.per, mid) <= i) lo = mid;
+          else hi = mid;
         }
-      });
-      SHB_CUDA(cudaMemcpyAsync(static_cast<char*>(a.dst->ptr) + p0 * a.bytes, out, (p1 - p0) * a.bytes,
+        for (size_t g = lo; i < end; ++g) {
+          const size_t in = i - first_of(a.per, g), n = std::min(end - i, count_of(a.per, g) - in);
+          if (n) fill(sg->kind, g, in, n, base + sg->at + (i - sg->first) * a.bytes);
+          i += n;
+        }
+      }
+    });
+  };
+  auto send = [&]() -> shb_status {
+    char* base = staging.ptr + half * cap;
+    SHB_CUDA(cudaEventSynchronize(done[half].e));  // (returns at once before the first record)
+    fill_piece(base);
+    for (const Segment& g : piece) {
+      const size_t bytes = arrays[g.kind].bytes;
+      SHB_CUDA(cudaMemcpyAsync(arrays[g.kind].dst->as<char>() + g.first * bytes, base + g.at, g.n * bytes,
                                cudaMemcpyHostToDevice, st));
-      SHB_CUDA(cudaEventRecord(done[half].e, st));
+    }
+    SHB_CUDA(cudaEventRecord(done[half].e, st));
+    half ^= 1;
+    used = 0;
+    piece.clear();
+    return SHB_OK;
+  };
+  for (int k = 0; k < KINDS; ++k) {
+    const size_t all = count(arrays[k].per), bytes = arrays[k].bytes;
+    for (size_t first = 0; first < all;) {
+      const size_t n = std::min(all - first, (cap - used) / bytes);
+      if (n) piece.push_back(Segment{(Kind)k, first, n, used});
+      first += n;
+      used += padded(n * bytes);
+      if (first < all) SHB_TRY(send());
     }
   }
-  return SHB_OK;
+  return piece.empty() ? SHB_OK : send();
 }
 
 static shb_status bad(const std::string& m) {

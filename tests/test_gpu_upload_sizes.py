@@ -1,7 +1,8 @@
 """Scene uploads around the size of the staging buffer that a context keeps
-(64 MiB of host memory): what fits is laid out whole, more goes through the
-buffer's halves in pieces that cut geometries anywhere.  Most of the vertices
-belong to no triangle, so that the oracle and the tree stay small."""
+(32 MiB of page-locked host memory): what fits is laid out whole, more goes
+through the buffer's halves in pieces that cut arrays and geometries anywhere.
+Most of the vertices belong to no triangle, so that the oracle and the tree
+stay small."""
 import ctypes as C
 import time
 
@@ -37,10 +38,10 @@ def big(sizes, seed=1):
 
 
 @pytest.mark.parametrize("sizes", [
-    [64 * 2 ** 20 // VERTEX - 20_000],         # a little less than the buffer
-    [64 * 2 ** 20 // VERTEX + 20_000],         # a little more
+    [32 * 2 ** 20 // VERTEX - 10_000],         # a little less than the buffer
+    [32 * 2 ** 20 // VERTEX + 10_000],         # a little more
     [3, 0, 700_001, 0, 0, 900_000, 1, 5, 0],
-    [2_796_202, 1, 3_000_000],                 # a half of the vertices (12 bytes each) and one less
+    [1_398_101, 1, 1_500_000],                 # the positions that a half holds, and one more
     [n for k in range(2000) for n in (k % 7, 1500)],
 ])
 def test_contents(gpu_ctx, sizes):
@@ -63,7 +64,7 @@ def test_time_grows_with_the_bytes(gpu_ctx):
     # twice the bytes across the buffer's size: three times the time is
     # generous; in plain memory of its own the larger one took about ten times
     ms = []
-    for n in (900_000, 1_800_000):
+    for n in (450_000, 900_000, 1_800_000):
         desc, keep = pack_scene(big([n]))
         ts = []
         for _ in range(6):
@@ -73,4 +74,29 @@ def test_time_grows_with_the_bytes(gpu_ctx):
             ts.append(time.perf_counter() - t)
             gpu_ctx.lib.shb_scene_destroy(h)
         ms.append(min(ts) * 1e3)
-    assert ms[1] < 3 * ms[0], ms
+    assert ms[1] < 3 * ms[0] and ms[2] < 3 * ms[1], ms
+
+
+def locked():
+    """Bytes of shared memory this process holds, as which the driver's
+    page-locked host memory counts."""
+    return int(next(x for x in open("/proc/self/status") if x.startswith("RssShmem:")).split()[1]) << 10
+
+
+@pytest.mark.parametrize("vertices,kept", [(1_000, 2 << 20), (300_000, 300_000 * VERTEX * 9 // 8 + (1 << 20)),
+                                           (900_000, 32 << 20), (1_800_000, 32 << 20)])
+def test_first_upload_locks_no_more_than_it_needs(vertices, kept):
+    # A context's first upload waits until its staging buffer is locked, about
+    # 0.6 ms per MiB: what the upload needs and an eighth, at most 32 MiB (the
+    # driver rounds to 2 MiB).
+    from sh_baker_b200 import Context
+    desc, keep = pack_scene(big([vertices]))
+    ctx = Context()
+    before = locked()
+    h = C.c_void_p()
+    assert ctx.lib.shb_scene_upload(ctx.h, C.byref(desc), C.byref(h)) == 0
+    ctx.lib.shb_scene_destroy(h)
+    grown = locked() - before
+    ctx.close()
+    assert 0 < grown <= kept + (2 << 20)
+    assert locked() < before + grown  # given back with the context
