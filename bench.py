@@ -614,7 +614,7 @@ def run_exr(args):
     print(json.dumps(line), flush=True)
 
 
-def roofline_of(stats, steps, scene, w, ms, clk):
+def roofline_of(stats, traced, steps, scene, w, ms, clk):
     """Roofline of the dominant traversal kernel.  Traversal of incoherent
     rays is bound by instruction issue (dependent node fetches hit L1/L2,
     ncu shows ~80 % issue activity and DRAM traffic < 10 % of the model's
@@ -622,15 +622,16 @@ def roofline_of(stats, steps, scene, w, ms, clk):
     small case of the same scene) x rays traced / kernel time, against the
     SMs' issue slots (SMs x 4 schedulers x median SM clock under load).  The
     model-byte HBM figure (the algorithmic bytes of bytes_per_ray over the
-    measured copy bandwidth) is kept beside it as `hbm_model`."""
+    measured copy bandwidth) is kept beside it as `hbm_model`.  `traced` is
+    the any-hit rays traced in the steps (the stats count light queries, of
+    which samples of a texel share rays)."""
     import torch
     ext_ms = sum(s.extend_kernel_ms for s in stats)
     sh_ms = sum(s.shadow_kernel_ms for s in stats)
     ext_rays = sum(s.extend_rays for s in stats)
-    sh_rays = sum(s.shadow_rays for s in stats)
     bpr = bytes_per_ray(scene.triangle_count)
     dom = "closest_hit" if ext_ms >= sh_ms else "any_hit"
-    k_ms, k_rays = (ext_ms, ext_rays) if dom == "closest_hit" else (sh_ms, sh_rays)
+    k_ms, k_rays = (ext_ms, ext_rays) if dom == "closest_hit" else (sh_ms, traced)
     k_launch = sum((s.extend_launches if dom == "closest_hit" else s.shadow_launches) for s in stats)
     rays_per_launch = k_rays / max(k_launch, 1)
     hbm_achieved = k_rays * bpr / (k_ms / 1e3) / 1e9 if k_ms > 0 else 0.0
@@ -646,7 +647,7 @@ def roofline_of(stats, steps, scene, w, ms, clk):
             "rays_per_launch": rays_per_launch, "launch_ms": k_ms / max(k_launch, 1),
             "kernel_ms": {"closest_hit": ext_ms / steps, "any_hit": sh_ms / steps,
                           "shade": sum(s.shade_kernel_ms for s in stats) / steps},
-            "rays_per_s": (ext_rays + sh_rays) / (ms / 1e3),
+            "rays_per_s": (ext_rays + traced) / (ms / 1e3),
             "hbm_model": {"bytes_per_ray": bpr, "achieved": hbm_achieved, "peak": peak, "unit": "GB/s",
                           "frac": hbm_achieved / peak, "peak_source": peak_kind}}
     if prof:
@@ -785,7 +786,7 @@ def main():
         dist.barrier()
     clocks = ClockSampler(local)
     clocks.start()
-    launches0 = ctx.kernel_launches()
+    launches0, traced0 = ctx.kernel_launches(), ctx.shadow_rays_traced()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     torch.cuda.synchronize()
     ev0.record(stream)
@@ -794,12 +795,13 @@ def main():
     torch.cuda.synchronize()
     ms = ev0.elapsed_time(ev1)
     launches = ctx.kernel_launches() - launches0
+    traced = ctx.shadow_rays_traced() - traced0
     clk = clocks.stop()
     ts = sum(s.texel_samples for s in stats)
     ms, ts, value = job_rate(ms, ts, dist)
-    roof = roofline_of(stats, args.steps, scene, w, ms, clk)
+    roof = roofline_of(stats, traced, args.steps, scene, w, ms, clk)
     ext_rays = sum(s.extend_rays for s in stats)
-    sh_rays = sum(s.shadow_rays for s in stats)
+    queries = sum(s.shadow_rays for s in stats)
 
     # end to end through the public API from pinned host memory
     e2e = None
@@ -851,9 +853,9 @@ def main():
                 "traversal_per_step": {
                     "closest_hit": {"rays": ext_rays // args.steps,
                                     "launches": sum(s.extend_launches for s in stats) // args.steps},
-                    "any_hit": {"rays": sh_rays // args.steps,
+                    "any_hit": {"rays": traced // args.steps, "light_queries": queries // args.steps,
                                 "launches": sum(s.shadow_launches for s in stats) // args.steps}},
-                "rays_per_texel_sample": (ext_rays + sh_rays) / max(ts, 1)}
+                "rays_per_texel_sample": (ext_rays + traced) / max(ts, 1)}
     del sh, env
     g.close()
     ds.close()

@@ -189,7 +189,9 @@ typedef struct shb_bake_stats {
   uint64_t texel_samples;  /* valid texels x samples                      */
   uint64_t valid_texels;
   uint64_t extend_rays;    /* closest-hit rays traced                     */
-  uint64_t shadow_rays;    /* light queries (samples may share a ray)     */
+  uint64_t shadow_rays;    /* light queries; samples of a texel may share
+                              one any-hit ray (see
+                              shb_context_shadow_rays_traced)             */
   uint64_t kernel_launches;
   uint32_t error_flags;    /* device-side bounded-failure flags (0 = ok)  */
   uint32_t waves;
@@ -244,6 +246,10 @@ SHB_API shb_status shb_context_set_stream(shb_context* ctx, void* stream);
 SHB_API shb_status shb_context_synchronize(shb_context* ctx);
 /* Number of kernels this context has launched so far. */
 SHB_API uint64_t shb_context_kernel_launches(const shb_context* ctx);
+/* Number of any-hit rays the context's bakes and backward passes have traced
+ * so far: the light queries of shb_bake_stats.shadow_rays less those that
+ * shared the ray of another sample of their texel. */
+SHB_API uint64_t shb_context_shadow_rays_traced(const shb_context* ctx);
 
 /* Uploads the scene and builds the GPU BVH (binned SAH, compressed 8-wide
  * nodes).  Replaces BuildBVH (src/scene.cpp:209-262); the reference builds

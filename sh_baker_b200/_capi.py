@@ -140,6 +140,7 @@ SIGNATURES = {
     "shb_context_set_stream": (C.c_int, [vp, vp]),
     "shb_context_synchronize": (C.c_int, [vp]),
     "shb_context_kernel_launches": (C.c_uint64, [vp]),
+    "shb_context_shadow_rays_traced": (C.c_uint64, [vp]),
     "shb_scene_upload": (C.c_int, [vp, C.POINTER(SceneDesc), C.POINTER(vp)]),
     "shb_scene_destroy": (C.c_int, [vp]),
     "shb_scene_rebuild_bvh": (C.c_int, [vp]),

@@ -75,6 +75,11 @@ class Context:
     def kernel_launches(self) -> int:
         return int(self.lib.shb_context_kernel_launches(self.h))
 
+    def shadow_rays_traced(self) -> int:
+        """Any-hit rays traced so far; BakeStats.shadow_rays counts the light
+        queries, of which samples of one texel may share a ray."""
+        return int(self.lib.shb_context_shadow_rays_traced(self.h))
+
     def set_stream(self, stream_ptr: int) -> None:
         A.check(self.lib.shb_context_set_stream(self.h, C.c_void_p(stream_ptr)))
 

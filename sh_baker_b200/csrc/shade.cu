@@ -875,9 +875,8 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
       __stcs(a.ext[0].d + p, make_float4(dw.x, dw.y, dw.z, __uint_as_float(1u)));
     }
   }
-  // shadow_rays counts the light queries, shared or not
   if (!BWD && lane == 0 && shared_rays)
-    atomicAdd(&a.c64->shadow_rays, (unsigned long long)shared_rays);
+    atomicAdd(&a.c64->shared_queries, (unsigned long long)shared_rays);
 }
 
 // --------------------------------------------------------------- shade ---
@@ -1838,11 +1837,12 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
   count_launch(c, launches);
   SHB_CUDA(cudaGetLastError());
   int err = 0;
-  Counters64 h64{0, 0};
+  Counters64 h64{0, 0, 0};
   SHB_CUDA(cudaMemcpyAsync(&err, cnt + CNT_ERROR, sizeof(int), cudaMemcpyDeviceToHost, st));
   SHB_CUDA(cudaMemcpyAsync(&h64, c64, sizeof(Counters64), cudaMemcpyDeviceToHost, st));
   if (c->profiling) cudaEventRecord(t_end, st);
   SHB_CUDA(cudaStreamSynchronize(st));
+  c->shadow_rays_traced += h64.shadow_rays;
   double ext_ms = 0.0, sh_ms = 0.0, shade_ms = 0.0;
   float total_ms = 0.f;
   if (c->profiling) {
@@ -1868,7 +1868,7 @@ shb_status bake_batch_device(shb_context* c, const std::vector<BakeSpec>& specs,
     stats->texel_samples = ts;
     stats->valid_texels = vt;
     stats->extend_rays = h64.extend_rays;
-    stats->shadow_rays = h64.shadow_rays;
+    stats->shadow_rays = h64.shadow_rays + h64.shared_queries;
     stats->error_flags = (uint32_t)err;
     stats->waves = (uint32_t)waves.size();
     stats->trace_ms = total_ms;

@@ -697,6 +697,8 @@ shb_status shb_context_synchronize(shb_context* ctx) {
 
 uint64_t shb_context_kernel_launches(const shb_context* ctx) { return ctx ? ctx->launches : 0; }
 
+uint64_t shb_context_shadow_rays_traced(const shb_context* ctx) { return ctx ? ctx->shadow_rays_traced : 0; }
+
 shb_status shb_rotation_part(const float transform[12], float rotation[9]) {
   return ::shb::guarded("shb_rotation_part", [&]() -> shb_status {
     if (!transform || !rotation) return bad("NULL argument");

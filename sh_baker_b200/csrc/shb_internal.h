@@ -266,6 +266,7 @@ struct shb_context {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   uint64_t launches = 0;
+  uint64_t shadow_rays_traced = 0;  // by all bakes and backward passes so far
   // scratch reused across calls
   shb::DevBuf scratch[28];
   shb::DevBuf counters;

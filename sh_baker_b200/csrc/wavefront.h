@@ -65,7 +65,8 @@ enum ErrorBits : int { ERR_STACK = 1, ERR_QUEUE = 2, ERR_ITER = 4 };
 
 struct Counters64 {
   unsigned long long extend_rays;
-  unsigned long long shadow_rays;
+  unsigned long long shadow_rays;    // any-hit rays traced
+  unsigned long long shared_queries; // light queries that share another's ray
 };
 
 // One bake of a batch (device table entry).  A single BakeSHLightMap call
