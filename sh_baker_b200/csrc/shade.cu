@@ -298,13 +298,16 @@ __device__ LightEval eval_light(const SceneView& sc, const DLight* lights, uint3
 // One light pick of the discrete distribution over weights (the counter
 // stream's uniform `u` against the running float sum; zero-weight lights
 // are never picked).
-// The running sums of up to kWeightCache lights are kept from the summing
-// pass in `cum`.  They never fall unless a light is negative
-// (SceneView::negative_lights), so the pick is a binary search over them;
-// sums that may fall are searched in order.  The weights are evaluated again
-// only for longer tables and when no sum exceeds the target (a uniform next
-// to 1, an overflow).  In each case the picked light is evaluated once, after
-// the search, for all lanes at once.
+// For up to kWeightCache lights the summing pass leaves in `cum` the largest
+// of the running sums so far: the sums themselves unless a light is negative,
+// and the first sum above the target is the first such maximum above it either
+// way, so the pick is a binary search.  The weights are evaluated again in
+// order only for longer tables and when no sum exceeds the target (a uniform
+// next to 1, an overflow).  In each case the picked light is evaluated once,
+// after the search, for all lanes at once.
+// (512^2 room, 24 lights, one of them negative: shading 6.9 ms, as without it;
+// 12.3 when its picks evaluated the lights in order, 7.5 with the sums
+// searched in order.  The maximum costs 0.4 % of k_nee's instructions.)
 // `lights` is the bake's light table in global memory or the block's copy
 // of it in shared memory.
 constexpr uint32_t kWeightCache = 32;
@@ -321,13 +324,9 @@ __device__ __forceinline__ bool pick_light(const SceneView& sc, const DLight* li
   int pick = -1;
   if (sc.light_count <= kWeightCache) {
     uint32_t pos = 0;
-    if (!sc.negative_lights) {
 #pragma unroll
-      for (uint32_t step = kWeightCache / 2; step > 0; step >>= 1)
-        if (pos + step < sc.light_count && !(target < cum[pos + step - 1])) pos += step;
-    } else {
-      while (pos + 1 < sc.light_count && !(target < cum[pos])) ++pos;
-    }
+    for (uint32_t step = kWeightCache / 2; step > 0; step >>= 1)
+      if (pos + step < sc.light_count && !(target < cum[pos + step - 1])) pos += step;
     if (target < cum[pos]) pick = (int)pos;
   }
   if (pick < 0) {
@@ -453,21 +452,23 @@ __device__ __forceinline__ uint32_t next_weights(const SceneView& sc, const DLig
 
 __device__ __forceinline__ float behind_margin(f3 N) { return 1e-5f * (fabsf(N.x) + fabsf(N.y) + fabsf(N.z)); }
 
-// Sum of all weights in light order; `cum` receives the running sums.
+// Sum of all weights in light order; `cum` receives the largest running sums.
 template <int AREA, bool HIT>
 __device__ __forceinline__ float light_weight_sum(const SceneView& sc, const DLight* lights, f3 P, f3 N, Event& ev,
                                                   bool wo_back, f3 aop, float* cum) {
-  float sum = 0.0f;
+  float sum = 0.0f, top = -INFINITY;
   const bool cached = sc.light_count <= kWeightCache;
   const float nm = behind_margin(N);
   for (uint32_t i = 0; i < sc.light_count;) {
     float wa, wb;
     const uint32_t k = next_weights<AREA, HIT>(sc, lights, i, P, N, nm, ev, wo_back, aop, wa, wb);
     sum += wa;
-    if (cached) cum[i] = sum;
+    top = fmaxf(top, sum);
+    if (cached) cum[i] = top;
     if (k == 2u) {
       sum += wb;
-      if (cached) cum[i + 1] = sum;
+      top = fmaxf(top, sum);
+      if (cached) cum[i + 1] = top;
     }
     i += k;
   }
@@ -777,6 +778,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
                              ? eval_light<AREA_NONE, false>(BL->sc, ll, (uint32_t)lane, Pl, Nl, ev, true, zero3).w
                              : 0.f;
       const float nm = behind_margin(N);
+      float top = -INFINITY;
       for (uint32_t i = 0; i < nl;) {
         float wa = 0.f, wb = 0.f;
         uint32_t k = 1;
@@ -792,10 +794,12 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
           k = __all_sync(0xFFFFFFFFu, !active || k == 2u) ? 2u : 1u;
         }
         sum += wa;
-        cum[i] = sum;
+        top = fmaxf(top, sum);
+        cum[i] = top;
         if (k == 2u) {
           sum += wb;
-          cum[i + 1] = sum;
+          top = fmaxf(top, sum);
+          cum[i + 1] = top;
         }
         i += k;
       }

@@ -182,15 +182,12 @@ void srgb_upload(const float table[256]);
 // * emission with the float products get_emission makes on the device.
 // Point lights: intensity * color.
 void light_consts(shb_scene* s) {
-  s->negative_lights = 0;
   for (uint32_t l = 0; l < s->light_count; ++l) {
     DLight& L = s->h_lights[l];
     L.emis_const = 0;
     L.er = L.eg = L.eb = 0.f;
     L.pair = PAIR_NONE;
     L.grey = 0;
-    for (float c : {L.cr, L.cg, L.cb})
-      if (L.type != SHB_LIGHT_AREA && !(L.intensity * c >= 0.f)) s->negative_lights = 1;
     if (L.type == SHB_LIGHT_POINT) {
       L.er = L.intensity * L.cr;
       L.eg = L.intensity * L.cg;
@@ -587,7 +584,6 @@ SceneView shb_scene::view() const {
   v.prim_count = prim_count;
   v.vertex_count = vertex_count;
   v.has_alpha = has_alpha;
-  v.negative_lights = negative_lights;
   return v;
 }
 

@@ -248,8 +248,7 @@ struct SceneView {
   const float4* area_tris;  // 4 per area-light triangle (shade.cu sample_area)
   uint32_t geom_count, mat_count, light_count, area_light_count;
   uint32_t prim_count, vertex_count;
-  int32_t has_alpha;        // any material with 4-channel albedo
-  int32_t negative_lights;  // a light's intensity * color has a negative channel
+  int32_t has_alpha;     // any material with 4-channel albedo
 };
 
 }  // namespace shb
@@ -286,7 +285,6 @@ struct shb_scene {
   uint32_t vertex_count = 0, prim_count = 0, geom_count = 0, mat_count = 0, light_count = 0;
   uint32_t area_light_count = 0;
   int32_t has_alpha = 0;
-  int32_t negative_lights = 0;
   int area_kind = shb::AREA_NONE;
   bool raster_ready = true;  // every geometry has normals, tangents, lightmap uvs
   std::string raster_error;

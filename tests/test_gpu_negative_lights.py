@@ -1,9 +1,8 @@
 """A table with a negative light (a fill that takes light away), whose running
-sums may fall: the pick searches them in order, and evaluates no light again.
-One light of 24 made slightly negative changes the work by that search alone,
-a look at up to 24 sums beside 24 light evaluations; the bound of a third
-more shading time leaves room for it (a second light loop per pick took
-three quarters more)."""
+sums may fall: the pick still searches them, and evaluates no light again.
+One light of 24 made slightly negative changes no work, at most the sums'
+search; the bound of a third more shading time leaves room for that (a second
+light loop per pick took three quarters more)."""
 import numpy as np
 import pytest
 
