@@ -779,29 +779,25 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
                              : 0.f;
       const float nm = behind_margin(N);
       float top = -INFINITY;
-      for (uint32_t i = 0; i < nl;) {
-        float wa = 0.f, wb = 0.f;
-        uint32_t k = 1;
+      // Every lane takes every i, so that all meet the shuffle: the second light
+      // of a pair is weighed with the first by the lanes that could take both,
+      // and by itself by those whose sampled distances were out of
+      // pair_weights' range.
+      float wb = 0.f;
+      bool have_b = false;
+      for (uint32_t i = 0; i < nl; ++i) {
+        float wa = wb;
         if (!AREA || ll[i].type != SHB_LIGHT_AREA) {
           wa = __shfl_sync(0xFFFFFFFFu, mine, (int)i);
-        } else {
+        } else if (!have_b) {
           // inactive lanes evaluate too (their weights are dropped below)
-          k = next_weights<AREA, false>(BL->sc, ll, i, P0, N, nm, ev, true, zero3, wa, wb);
-          // The lanes sample points of their own, and one that cannot take
-          // the pair (a distance out of pair_weights' range) has light i
-          // alone.  The step is the warp's, so that all lanes meet the
-          // shuffle above: the others weigh light i + 1 again.
-          k = __all_sync(0xFFFFFFFFu, !active || k == 2u) ? 2u : 1u;
+          have_b = next_weights<AREA, false>(BL->sc, ll, i, P0, N, nm, ev, true, zero3, wa, wb) == 2u;
+        } else {
+          have_b = false;
         }
         sum += wa;
         top = fmaxf(top, sum);
         cum[i] = top;
-        if (k == 2u) {
-          sum += wb;
-          top = fmaxf(top, sum);
-          cum[i + 1] = top;
-        }
-        i += k;
       }
       if (!active) sum = 0.f;
     } else if (active) {
