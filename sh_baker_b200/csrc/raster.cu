@@ -628,14 +628,15 @@ extern "C" SHB_API shb_status shb_dilate_noalloc(shb_context* ctx, int32_t kind,
     const int64_t n = (int64_t)width * height;  // width, height > 0 and < 2^31: no overflow
     const int ch = kind == SHB_DILATE_SH9 ? 27 : 1;
     const size_t esz = kind == SHB_DILATE_U8 ? 1 : 4;
-    auto too_large = [&](const std::string& need) {
-      set_error("shb_dilate_noalloc: " + std::to_string(width) + "x" + std::to_string(height) + " texels need " + need +
-                " bytes of scratch; the fixed array holds " + std::to_string(kNoAllocScratchBytes) +
-                " (about 153,000 texels of SH9, 3.3 M of float, 8.3 M of uint8)");
+    auto too_large = [&](const std::string& bytes) {
+      set_error("shb_dilate_noalloc: " + std::to_string(width) + "x" + std::to_string(height) +
+                " texels with their mask and flags are " + bytes + " bytes, more than the fixed array's " +
+                std::to_string(kNoAllocScratchBytes) +
+                " (about 153,000 texels of SH9, 3.3 M of float, 8.3 M of uint8 are taken)");
       return SHB_ERR_INVALID_ARG;
     };
-    // every texel needs at least one mask byte of scratch: bound n before the
-    // byte counts below are formed
+    // every texel has at least a mask byte: bound n before the byte counts
+    // below are formed
     if (n > (int64_t)kNoAllocScratchBytes) return too_large("more than " + std::to_string(n));
     const size_t pbytes = esz * (size_t)n * ch;
     const size_t pbytes_aligned = (pbytes + 255) & ~size_t(255);

@@ -311,11 +311,6 @@ __device__ LightEval eval_light(const SceneView& sc, const DLight* lights, uint3
 // `lights` is the bake's light table in global memory or the block's copy
 // of it in shared memory.
 constexpr uint32_t kWeightCache = 32;
-// Texel next-event estimation shares the punctual lights' weights across a
-// warp of one texel's samples also in scenes with area lights.
-#ifndef SHB_TEXEL_COOP_AREA
-#define SHB_TEXEL_COOP_AREA 1
-#endif
 
 template <int AREA, bool HIT, bool BWD = false>
 __device__ __forceinline__ bool pick_light(const SceneView& sc, const DLight* lights, f3 P, f3 N, Event& ev,
@@ -763,9 +758,8 @@ __global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAr
     const uint64_t key = active ? ((uint64_t)b << 32 | texel) : ~0ull;
     const int lead = act ? __ffs(act) - 1 : 0;
     const uint64_t key0 = __shfl_sync(0xFFFFFFFFu, key, lead);
-    const bool coop = act && __all_sync(0xFFFFFFFFu, !active || (key == key0 &&
-                                                                 (SHB_TEXEL_COOP_AREA || B->sc.area_light_count == 0) &&
-                                                                 B->sc.light_count <= kWeightCache));
+    const bool coop =
+        act && __all_sync(0xFFFFFFFFu, !active || (key == key0 && B->sc.light_count <= kWeightCache));
     if (coop) {
       const BakeItem* BL = a.bakes + (uint32_t)(key0 >> 32);
       const f3 Pl = {__shfl_sync(0xFFFFFFFFu, P0.x, lead), __shfl_sync(0xFFFFFFFFu, P0.y, lead),

@@ -596,6 +596,9 @@ __device__ __forceinline__ void consume(CoopWarp<SHADOW>& s, const PermTable& pe
       }
     }
   }
+  // Never taken: a lane whose ray has ended asks for another, and the refill that
+  // ends the loop finishes it.  Without the line the compiler's code for the
+  // closest hit is 1 % slower (263k triangles 82.8 -> 83.7 ms).
   if (ended >= 0) finish(ended, w, s.rec(lane), (ONE ? one : own).tris);
 }
 
