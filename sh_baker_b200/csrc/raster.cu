@@ -276,15 +276,20 @@ __global__ void k_mask_down(const uint8_t* __restrict__ in, int w, int h, int s,
 // per output row.  CH and S are the channels and the scale (0: any).  Bound
 // by HBM: every input float is read once.  With both known the S * S loads
 // of a thread are independent and in flight together and the texel index is
-// a 32-bit constant division: 3072^2 SH texels to 1024^2 in 210 us (5.4 TB/s;
-// 525 us with 64-bit divisions and a loop).
+// a 32-bit constant division.  The loops over outputs are not unrolled and the
+// registers are limited so that loads of enough warps are in flight: 1000^2 SH
+// texels from scale 2, 3 and 4 take 114, 203 and 283 us (left to the
+// compiler 341, 217 and 857, with 64-bit divisions and a loop 285, 494 and
+// 535; at scale 4 eight blocks 460, four with 16 loads each in flight less).
 template <int CH, int S>
-__global__ void __launch_bounds__(kThreads) k_downsample(const float* __restrict__ in, int in_w, int oh, int ow,
-                                                         int ch_, int s_, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads, CH != 27 ? 1 : S == 4 ? 4 : 8)
+    k_downsample(const float* __restrict__ in, int in_w, int oh, int ow, int ch_, int s_, float* __restrict__ out) {
   const int ch = CH ? CH : ch_, s = S ? S : s_;
   const int64_t row = (int64_t)ow * ch, stride = (int64_t)in_w * ch;
+#pragma unroll 1
   for (int64_t y = blockIdx.y; y < oh; y += gridDim.y) {
     const float* src = in + y * s * stride;
+#pragma unroll 1
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < row; i += (int64_t)gridDim.x * blockDim.x) {
       const int64_t x = CH ? (int64_t)((uint32_t)i / (uint32_t)CH) : i / ch;
       const float* p = src + x * (s * ch) + (i - x * ch);
