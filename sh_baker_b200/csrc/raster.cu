@@ -278,11 +278,11 @@ __global__ void k_mask_down(const uint8_t* __restrict__ in, int w, int h, int s,
 // of a thread are independent and in flight together and the texel index is
 // a 32-bit constant division.  The loops over outputs are not unrolled and the
 // registers are limited so that loads of enough warps are in flight: 1000^2 SH
-// texels from scale 2, 3 and 4 take 114, 203 and 283 us (left to the
+// texels from scale 2, 3 and 4 take 114, 200 and 283 us (left to the
 // compiler 341, 217 and 857, with 64-bit divisions and a loop 285, 494 and
 // 535; at scale 4 eight blocks 460, four with 16 loads each in flight less).
 template <int CH, int S>
-__global__ void __launch_bounds__(kThreads, CH != 27 ? 1 : S == 4 ? 4 : 8)
+__global__ void __launch_bounds__(kThreads, CH != 27 ? 1 : S == 4 ? 4 : S == 3 ? 6 : 8)
     k_downsample(const float* __restrict__ in, int in_w, int oh, int ow, int ch_, int s_, float* __restrict__ out) {
   const int ch = CH ? CH : ch_, s = S ? S : s_;
   const int64_t row = (int64_t)ow * ch, stride = (int64_t)in_w * ch;
