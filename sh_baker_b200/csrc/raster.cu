@@ -258,53 +258,69 @@ __global__ void k_validity(const shb_surface_point* __restrict__ pts, int64_t n,
     out[i] = pts[i].material_id >= 0;
 }
 
-// src/rasterizer.cpp:222-241, a block row per output row.
+// src/rasterizer.cpp:222-241; launched by Rows.  (A texel is done at its first
+// valid sample: without the exits 3 x 2^18 texels from scale 8, a third of them
+// valid, took 51 us, with them 19.)
 __global__ void k_mask_down(const uint8_t* __restrict__ in, int w, int h, int s, uint8_t* __restrict__ out) {
   const int64_t stride = (int64_t)w * s;
-  for (int64_t y = blockIdx.y; y < h; y += gridDim.y) {
-    const uint8_t* row = in + y * s * stride;
+  for (int64_t y = blockIdx.y * (int64_t)blockDim.y + threadIdx.y; y < h; y += (int64_t)gridDim.y * blockDim.y) {
+    const uint8_t* rows = in + y * s * stride;
     for (int64_t x = blockIdx.x * blockDim.x + threadIdx.x; x < w; x += gridDim.x * blockDim.x) {
       uint8_t any = 0;
-      for (int dy = 0; dy < s; ++dy)
-        for (int dx = 0; dx < s; ++dx) any |= row[dy * stride + x * s + dx] != 0;
+      for (int dy = 0; dy < s && !any; ++dy)
+        for (int dx = 0; dx < s; ++dx)
+          if (rows[dy * stride + x * s + dx]) {
+            any = 1;
+            break;
+          }
       out[y * w + x] = any;
     }
   }
 }
 
-// src/baker.cpp:151-182: one thread per (output texel, channel), a block row
-// per output row.  CH and S are the channels and the scale (0: any).  Bound
-// by HBM: every input float is read once.  With both known the S * S loads
-// of a thread are independent and in flight together and the texel index is
-// a 32-bit constant division.  The loops over outputs are not unrolled and the
-// registers are limited so that loads of enough warps are in flight: 1000^2 SH
-// texels from scale 2, 3 and 4 take 114, 200 and 283 us (left to the
-// compiler 341, 217 and 857, with 64-bit divisions and a loop 285, 494 and
-// 535; at scale 4 eight blocks 460, four with 16 loads each in flight less).
+// src/baker.cpp:151-182: one thread per (output texel, channel), launched by
+// Rows, with CH channels and scale S.  Bound by HBM: every input float is read
+// once, S * S independent loads of a thread in flight together.  All indices
+// but a row's address are 32 bits: with 64-bit ones the compiler's register
+// allocation decided how many loads were in flight, and the time of 1000^2 SH
+// texels swung between 114 and 341 us at scale 2, 200 and 411 at 3, 283 and
+// 857 at 4 (with a loop over the S * S texels 285, 494 and 535); now 104,
+// 162 and 275 us (5.2, 6.7 and 6.7 TB/s).
 template <int CH, int S>
-__global__ void __launch_bounds__(kThreads, CH != 27 ? 1 : S == 4 ? 4 : S == 3 ? 6 : 8)
-    k_downsample(const float* __restrict__ in, int in_w, int oh, int ow, int ch_, int s_, float* __restrict__ out) {
-  const int ch = CH ? CH : ch_, s = S ? S : s_;
-  const int64_t row = (int64_t)ow * ch, stride = (int64_t)in_w * ch;
+__global__ void __launch_bounds__(kThreads) k_downsample(const float* __restrict__ in, uint32_t stride, int oh,
+                                                         uint32_t row, float* __restrict__ out) {
+  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x, is = gridDim.x * blockDim.x;
+  const int ys = gridDim.y * blockDim.y;
 #pragma unroll 1
-  for (int64_t y = blockIdx.y; y < oh; y += gridDim.y) {
-    const float* src = in + y * s * stride;
+  for (int y = blockIdx.y * blockDim.y + threadIdx.y; y < oh; y += ys) {
+    const float* src = in + (int64_t)y * S * stride;
+    float* dst = out + (int64_t)y * row;
 #pragma unroll 1
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < row; i += (int64_t)gridDim.x * blockDim.x) {
-      const int64_t x = CH ? (int64_t)((uint32_t)i / (uint32_t)CH) : i / ch;
-      const float* p = src + x * (s * ch) + (i - x * ch);
+    for (uint32_t i = i0; i < row; i += is) {
+      const float* p = src + (i + i / (uint32_t)CH * (uint32_t)((S - 1) * CH));
+      float v[S * S], avg = 0.0f;
+#pragma unroll
+      for (int k = 0; k < S * S; ++k) v[k] = __ldg(p + (int64_t)(k / S) * stride + (k % S) * CH);
+#pragma unroll
+      for (int k = 0; k < S * S; ++k) avg += v[k];
+      dst[i] = avg * (1.f / float(S * S));
+    }
+  }
+}
+// Any channels and scale; I: uint32_t where an input row's floats fit 31 bits.
+template <class I>
+__global__ void __launch_bounds__(kThreads) k_downsample_any(const float* __restrict__ in, I stride, int64_t oh, I row,
+                                                             int ch, int s, float* __restrict__ out) {
+  const I i0 = blockIdx.x * blockDim.x + threadIdx.x, is = gridDim.x * blockDim.x;
+  for (int64_t y = blockIdx.y * blockDim.y + threadIdx.y; y < oh; y += gridDim.y * blockDim.y) {
+    const float* src = in + y * s * (int64_t)stride;
+    float* dst = out + y * (int64_t)row;
+    for (I i = i0; i < row; i += is) {
+      const float* p = src + (i + i / (I)ch * (I)(s - 1) * (I)ch);
       float avg = 0.0f;
-      if (S) {
-        float v[S ? S * S : 1];
-#pragma unroll
-        for (int k = 0; k < S * S; ++k) v[k] = __ldg(p + (k / (S ? S : 1)) * stride + (k % (S ? S : 1)) * ch);
-#pragma unroll
-        for (int k = 0; k < S * S; ++k) avg += v[k];
-      } else {
-        for (int dy = 0; dy < s; ++dy)
-          for (int dx = 0; dx < s; ++dx) avg += p[dy * stride + (int64_t)dx * ch];
-      }
-      out[y * row + i] = avg * (1.f / float(s * s));
+      for (int dy = 0; dy < s; ++dy)
+        for (int dx = 0; dx < s; ++dx) avg += p[dy * (int64_t)stride + (int64_t)dx * ch];
+      dst[i] = avg * (1.f / float(s * s));
     }
   }
 }
@@ -417,12 +433,22 @@ __global__ void __launch_bounds__(kThreads) k_dilate(T* __restrict__ px, uint8_t
   if (any) changed[pass - 1] = 1;
 }
 
-// A grid of block rows over a w x h texture.
-inline dim3 grid_rows(int64_t w, int64_t h) {
-  const int64_t gx = std::min<int64_t>((w + kThreads - 1) / kThreads, 1024);
-  const int64_t cap = std::max<int64_t>((int64_t)sm_count() * 256 / gx, 1);
-  return dim3((unsigned)gx, (unsigned)std::min<int64_t>(std::min<int64_t>(h, cap), 65535));
-}
+// A launch over the rows of a w x h texture: a block takes 256 elements of a
+// row or, where rows are shorter, several rows, so that its lanes are used
+// (with a row a block, 1 x 2^20 texels of one channel from scale 2 took 198 us, a
+// mask 280; now 13 and 16).
+struct Rows {
+  dim3 grid, block;
+  Rows(int64_t w, int64_t h) {
+    unsigned bx = 1;
+    while (bx < w && bx < (unsigned)kThreads) bx *= 2;
+    const unsigned by = kThreads / bx;
+    const int64_t gx = std::min<int64_t>((w + bx - 1) / bx, 1024);
+    const int64_t cap = std::max<int64_t>((int64_t)sm_count() * 256 / gx, 1);
+    block = dim3(bx, by);
+    grid = dim3((unsigned)gx, (unsigned)std::min<int64_t>({(h + by - 1) / by, cap, 65535}));
+  }
+};
 
 // Runs `passes` dilation passes with n labels and min(passes, kMaxLabel)
 // flags of scratch.
@@ -519,7 +545,8 @@ shb_status validity_mask_device(shb_context* c, const shb_surface_point* pts, in
 
 shb_status downsample_mask_device(shb_context* c, const uint8_t* in, int w, int h, int s, uint8_t* out) {
   if ((int64_t)w * h <= 0) return SHB_OK;
-  k_mask_down<<<grid_rows(w, h), kThreads, 0, c->stream>>>(in, w, h, s, out);
+  const Rows rows(w, h);
+  k_mask_down<<<rows.grid, rows.block, 0, c->stream>>>(in, w, h, s, out);
   count_launch(c);
   SHB_CUDA(cudaGetLastError());
   return SHB_OK;
@@ -532,17 +559,22 @@ shb_status downsample_device(shb_context* c, const float* in, int w, int h, int 
   }
   const int ow = w / s, oh = h / s;
   if ((int64_t)ow * oh * ch <= 0) return SHB_OK;
-  const dim3 grid = grid_rows((int64_t)ow * ch, oh);
-  auto run = [&](auto kernel) { kernel<<<grid, kThreads, 0, c->stream>>>(in, w, oh, ow, ch, s, out); };
-  // (the constant division is in 32 bits)
-  if ((int64_t)ow * ch > 0xFFFFFFFFll) run(k_downsample<0, 0>);
+  const int64_t row = (int64_t)ow * ch, stride = (int64_t)w * ch;
+  const Rows rows(row, oh);
+  auto run = [&](auto kernel) {
+    kernel<<<rows.grid, rows.block, 0, c->stream>>>(in, (uint32_t)stride, oh, (uint32_t)row, out);
+  };
+  if (stride > INT32_MAX)
+    k_downsample_any<int64_t><<<rows.grid, rows.block, 0, c->stream>>>(in, stride, oh, row, ch, s, out);
   else if (ch == 27 && s == 2) run(k_downsample<27, 2>);
   else if (ch == 27 && s == 3) run(k_downsample<27, 3>);
   else if (ch == 27 && s == 4) run(k_downsample<27, 4>);
   else if (ch == 1 && s == 2) run(k_downsample<1, 2>);
   else if (ch == 1 && s == 3) run(k_downsample<1, 3>);
   else if (ch == 1 && s == 4) run(k_downsample<1, 4>);
-  else run(k_downsample<0, 0>);
+  else
+    k_downsample_any<uint32_t><<<rows.grid, rows.block, 0, c->stream>>>(in, (uint32_t)stride, oh, (uint32_t)row, ch, s,
+                                                                        out);
   count_launch(c);
   SHB_CUDA(cudaGetLastError());
   return SHB_OK;
