@@ -337,10 +337,17 @@ __global__ void __launch_bounds__(kThreads) k_downsample_any(const float* __rest
 // on 85 % of the page: 1.9 -> 0.4 ms).
 constexpr uint16_t kUnfilled = 0xFFFFu;
 constexpr int kMaxLabel = 0xFFFE;  // passes per run of labels
+// Images of up to this many texels take a thread per float: 64^2 charts of
+// SH9, 4 passes 37 us (tiles 70), 128^2 180 (71); 384^2 charts of one float 45
+// (53), 512^2 142 (53).
+constexpr int64_t kFlatTexels = 160000, kFlatSh = 8192;
 
-__global__ void k_labels(const uint8_t* __restrict__ mask, int64_t n, uint16_t* __restrict__ label) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    label[i] = mask[i] ? 0 : kUnfilled;
+// The labels at the start of a run of passes, and its flags of change.
+__global__ void k_labels(const uint8_t* __restrict__ mask, int64_t n, uint16_t* __restrict__ label, int* changed,
+                         int run) {
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, is = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = i0; i < n; i += is) label[i] = mask[i] ? 0 : kUnfilled;
+  for (int64_t i = i0; i < run; i += is) changed[i] = 0;
 }
 
 // Bit (dy + 1) * 3 + (dx + 1) for each neighbour of texel (x, y) with a
@@ -356,32 +363,88 @@ __device__ __forceinline__ uint32_t filled_neighbours(const uint16_t* label, int
   return m;
 }
 
-// One pass.  Pass p is skipped when pass p - 1 filled nothing.  A warp looks
-// at 8 x 4 texels at a time, of which a straight front crosses few: with
-// several channels it fills them one after the other, a lane per channel, so
-// that a texel's floats are read and written together, and the longest such
-// chain is the pass's time (with 32 texels of a row per warp it was 20 us).
-constexpr int kTileW = kThreads / 32 * 8, kTileH = 16;
+// One pass.  Pass p is skipped when pass p - 1 filled nothing.
+
+// A thread per float: all CH threads of a texel find it open (a label of this
+// pass is one of them filling it).  Small images fill the device better this
+// way.
+template <class T, int CH>
+__global__ void __launch_bounds__(kThreads) k_dilate_flat(T* __restrict__ px, uint8_t* __restrict__ mask,
+                                                          uint16_t* __restrict__ label, uint32_t w, uint32_t h,
+                                                          int* changed, int pass) {
+  if (pass > 1 && *(volatile int*)(changed + pass - 2) == 0) return;
+  const uint32_t n = w * h * CH;  // below 2^31
+  bool any = false;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t t = i / CH;
+    if (label[t] < pass) continue;
+    const uint32_t y = t / w, x = t - y * w;
+    const uint32_t nb = filled_neighbours(label, (int)w, (int)h, (int)x, (int)y, pass);
+    if (!nb) continue;
+    T acc = T();
+    for (uint32_t m = nb; m; m &= m - 1) {
+      const int k = __ffs((int)m) - 1;
+      acc = (T)(acc + px[i + ((k / 3 - 1) * (int64_t)w + (k % 3 - 1)) * CH]);
+    }
+    px[i] = (T)(acc * (1.0f / __popc(nb)));
+    if (i - t * CH == 0) {
+      label[t] = (uint16_t)pass;
+      mask[t] = 1;
+      any = true;
+    }
+  }
+  if (any) changed[pass - 1] = 1;
+}
+
+// Tiles of a larger image.  A warp looks at 8 x 4 texels at a time, of which
+// a straight front crosses few: with several channels it fills them one after
+// the other, a lane per channel, so that a texel's floats are read and written
+// together, and the longest such chain is the pass's time (with 32 texels of a
+// row per warp it was 20 us).  Images of fewer columns or rows take narrower or
+// flatter tiles (with 8 x 4 and eight warps side by side, one column of 2^20
+// floats took 289 us a pass, now 31).
+struct DilateTile {
+  int lane_bits, warp_bits;  // log2 of a warp's lanes, and of a block's warps, side by side
+  int lanes, warps;          // the same counts
+  static constexpr int kRows = 4;  // tiles of a warp, one below the other
+  DilateTile(int64_t w, int64_t h) {
+    auto bits = [](int64_t n, int most) {  // log2 of the least power of two of at least n
+      int b = 0;
+      while (b < most && (int64_t(1) << b) < n) ++b;
+      return b;
+    };
+    lane_bits = w <= 4 ? bits(w, 2) : h == 1 ? 5 : h == 2 ? 4 : 3;
+    lanes = 1 << lane_bits;
+    warp_bits = bits((w + lanes - 1) / lanes, 3);
+    warps = 1 << warp_bits;
+  }
+  __host__ __device__ int width() const { return lanes * warps; }
+  __host__ __device__ int warp_height() const { return (32 >> lane_bits) * kRows; }
+  __host__ __device__ int height() const { return warp_height() * ((kThreads / 32) >> warp_bits); }
+};
+
 template <class T, int CH>
 __global__ void __launch_bounds__(kThreads) k_dilate(T* __restrict__ px, uint8_t* __restrict__ mask,
                                                      uint16_t* __restrict__ label, int w, int h, int* changed,
-                                                     int pass) {
+                                                     int pass, DilateTile tile) {
   if (pass > 1 && *(volatile int*)(changed + pass - 2) == 0) return;
-  const int lane = threadIdx.x & 31, lx = lane & 7, ly = lane >> 3;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bits = tile.lane_bits;
+  const int lx = lane & (tile.lanes - 1), ly = lane >> bits, lh = 32 >> bits;
+  const int wx = (warp & (tile.warps - 1)) << bits, wy = (warp >> tile.warp_bits) * tile.warp_height();
   bool any = false;
-  for (int64_t y0 = blockIdx.y * (int64_t)kTileH; y0 < h; y0 += gridDim.y * (int64_t)kTileH) {
-    for (int64_t x0 = blockIdx.x * (int64_t)kTileW + (threadIdx.x >> 5) * 8; x0 < w; x0 += gridDim.x * (int64_t)kTileW) {
+  for (int64_t y0 = blockIdx.y * (int64_t)tile.height() + wy; y0 < h; y0 += gridDim.y * (int64_t)tile.height()) {
+    for (int64_t x0 = blockIdx.x * (int64_t)tile.width() + wx; x0 < w; x0 += gridDim.x * (int64_t)tile.width()) {
       const int64_t x = x0 + lx;
-      bool open[kTileH / 4];
+      bool open[DilateTile::kRows];
 #pragma unroll
-      for (int r = 0; r < kTileH / 4; ++r) {
-        const int64_t y = y0 + 4 * r + ly;
+      for (int r = 0; r < DilateTile::kRows; ++r) {
+        const int64_t y = y0 + lh * r + ly;
         open[r] = x < w && y < h && label[y * w + x] == kUnfilled;
       }
 #pragma unroll
-      for (int r = 0; r < kTileH / 4; ++r) {
+      for (int r = 0; r < DilateTile::kRows; ++r) {
         if (!__any_sync(0xFFFFFFFFu, open[r])) continue;
-        const int64_t y = y0 + 4 * r + ly, t = y * w + x;
+        const int64_t y = y0 + lh * r + ly, t = y * w + x;
         const uint32_t nb = open[r] ? filled_neighbours(label, w, h, (int)x, (int)y, pass) : 0u;
         if (CH == 1) {
           if (nb) {
@@ -405,7 +468,7 @@ __global__ void __launch_bounds__(kThreads) k_dilate(T* __restrict__ px, uint8_t
               lnb[q] = __shfl_sync(0xFFFFFFFFu, nb, l);
               if (!todo) lnb[q] = 0u;
               todo &= todo - 1;
-              lt[q] = (y0 + 4 * r + (l >> 3)) * w + x0 + (l & 7);
+              lt[q] = (y0 + lh * r + (l >> bits)) * w + x0 + (l & (tile.lanes - 1));
 #pragma unroll
               for (int k = 0; k < 9; ++k)
                 v[q][k] = lane < CH && ((lnb[q] >> k) & 1u)
@@ -456,20 +519,23 @@ shb_status dilate_passes(shb_context* c, int kind, int w, int h, void* pixels, u
                          uint16_t* label, int* changed) {
   cudaStream_t st = c->stream;
   const int64_t n = (int64_t)w * h;
-  const dim3 grid((unsigned)std::min<int64_t>(((int64_t)w + kTileW - 1) / kTileW, 4096),
-                  (unsigned)std::min<int64_t>(((int64_t)h + kTileH - 1) / kTileH, 4096));
+  const DilateTile tile(w, h);
+  const dim3 grid((unsigned)std::min<int64_t>(((int64_t)w + tile.width() - 1) / tile.width(), 4096),
+                  (unsigned)std::min<int64_t>(((int64_t)h + tile.height() - 1) / tile.height(), 4096));
+  const int ch = kind == SHB_DILATE_SH9 ? 27 : 1;
+  const bool flat = n <= (ch == 1 ? kFlatTexels : kFlatSh);
   for (int done = 0; done < passes;) {
     const int run = std::min(passes - done, kMaxLabel);
-    SHB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int) * (size_t)run, st));
-    k_labels<<<grid_for(n), kThreads, 0, st>>>(mask, n, label);
-    for (int p = 1; p <= run; ++p) {
-      if (kind == SHB_DILATE_U8)
-        k_dilate<uint8_t, 1><<<grid, kThreads, 0, st>>>((uint8_t*)pixels, mask, label, w, h, changed, p);
-      else if (kind == SHB_DILATE_F32)
-        k_dilate<float, 1><<<grid, kThreads, 0, st>>>((float*)pixels, mask, label, w, h, changed, p);
-      else
-        k_dilate<float, 27><<<grid, kThreads, 0, st>>>((float*)pixels, mask, label, w, h, changed, p);
-    }
+    k_labels<<<grid_for(std::max<int64_t>(n, run)), kThreads, 0, st>>>(mask, n, label, changed, run);
+    auto pass = [&](auto tiles, auto flat_one, auto* px) {
+      for (int p = 1; p <= run; ++p) {
+        if (flat) flat_one<<<grid_for(n * ch), kThreads, 0, st>>>(px, mask, label, (uint32_t)w, (uint32_t)h, changed, p);
+        else tiles<<<grid, kThreads, 0, st>>>(px, mask, label, w, h, changed, p, tile);
+      }
+    };
+    if (kind == SHB_DILATE_U8) pass(k_dilate<uint8_t, 1>, k_dilate_flat<uint8_t, 1>, (uint8_t*)pixels);
+    else if (kind == SHB_DILATE_F32) pass(k_dilate<float, 1>, k_dilate_flat<float, 1>, (float*)pixels);
+    else pass(k_dilate<float, 27>, k_dilate_flat<float, 27>, (float*)pixels);
     count_launch(c, (uint64_t)run + 1);
     done += run;
   }

@@ -65,3 +65,23 @@ def test_thin_masks(timed, w):
     square, thin = (timed(lambda c: c.lib.shb_downsample_validity_mask(c.h, m.data_ptr(), a, n // a, 2, out.data_ptr(), 1))
                     for a in (1024, w))
     assert thin < 2.5 * square + 5.0, (square, thin)
+
+
+@pytest.mark.parametrize("ch", [1, 5, 27])
+def test_short_rows_match_oracle(ch):
+    # several rows a block, up to and beyond its 256 elements
+    import numpy as np
+
+    from oracle import pyoracle as O
+    from sh_baker_b200 import api
+    ctx = Context()
+    rng = np.random.default_rng(ch)
+    for w, h in ((1, 4001), (2, 777), (3, 1000), (9, 95), (10, 33), (51, 40), (52, 41), (255, 9), (257, 5), (600, 3)):
+        for s in (2, 3, 4, 5):
+            x = rng.normal(size=(h * s + s // 2, w * s + 1, ch)).astype(np.float32)
+            got = api._downsample(x, x.shape[1], x.shape[0], ch, s, ctx)
+            assert got.tobytes() == O.downsample(x, x.shape[1], x.shape[0], ch, s).astype(np.float32).tobytes(), (w, h, s)
+        m = (rng.random((h * 3, w * 3)) < 0.1).astype(np.uint8)
+        want = m.reshape(h, 3, w, 3).max(axis=(1, 3))
+        assert np.array_equal(api.DownsampleValidityMask(m, w, h, 3, ctx=ctx).reshape(h, w), want)
+    ctx.close()
