@@ -38,11 +38,12 @@ constexpr int kThreads = 256;
 // - k_nee: 3 where area lights are weighed in pairs (the pair's records need
 //   the registers: shading of the 768^2 atrium 120.6 ms at 4, 117.6 at 3),
 //   else 4 (cut-out room 6.28 against 6.35 ms);
-// - k_generate: 3 without area lights, else 2 (atrium 114.9 ms, 117.7
-//   unbounded, 122.1 at 3; room and quad equal at 2 and 3, slower at 4);
+// - k_generate: 2 where area lights are weighed in pairs (atrium 114.9 ms,
+//   117.7 unbounded, 122.1 at 3), else 3 (40 textured emitters, 256^2, no
+//   bounces: 1.54 ms, at 2 1.68; room and quad equal at 2 and 3, slower at 4);
 // - the adjoint's kernels: 2, at 1 the backward pass ran 14 % slower.
 constexpr int kShadeBlocks = 4, kFusedBlocks = 4, kNeePairBlocks = 3, kNeeBlocks = 4, kGenBlocks = 3,
-              kGenAreaBlocks = 2, kAdjointBlocks = 2;
+              kGenPairBlocks = 2, kAdjointBlocks = 2;
 // Alpha branches per path kept apart for deterministic accumulation: the
 // wave is shrunk by 2^min(bounces, kMaxBranchLog).  Branch slots beyond that
 // (more than six transmissive bounces) fall back to atomic accumulation.
@@ -303,8 +304,10 @@ __device__ LightEval eval_light(const SceneView& sc, const DLight* lights, uint3
 // and the first sum above the target is the first such maximum above it either
 // way, so the pick is a binary search.  The weights are evaluated again in
 // order only for longer tables and when no sum exceeds the target (a uniform
-// next to 1, an overflow).  In each case the picked light is evaluated once,
-// after the search, for all lanes at once.
+// next to 1, an overflow).  The search's light is evaluated for all lanes at
+// once, by the code that evaluates the scan's: with a place of its own the
+// kernels of area lights spilled more (atrium, shading 111.5 ms, now 109.7)
+// and long tables evaluated the picked light twice.
 // (512^2 room, 24 lights, one of them negative: shading 6.9 ms, as without it;
 // 12.3 when its picks evaluated the lights in order, 7.5 with the sums
 // searched in order.  The maximum costs 0.4 % of k_nee's instructions.)
@@ -316,31 +319,42 @@ template <int AREA, bool HIT, bool BWD = false>
 __device__ __forceinline__ bool pick_light(const SceneView& sc, const DLight* lights, f3 P, f3 N, Event& ev,
                                            bool wo_back, f3 aop, float sum, float u, const float* cum, LightEval& out) {
   const float target = u * sum;
-  int pick = -1;
+  bool found = false;
+  uint32_t i = 0;
   if (sc.light_count <= kWeightCache) {
-    uint32_t pos = 0;
 #pragma unroll
     for (uint32_t step = kWeightCache / 2; step > 0; step >>= 1)
-      if (pos + step < sc.light_count && !(target < cum[pos + step - 1])) pos += step;
-    if (target < cum[pos]) pick = (int)pos;
+      if (i + step < sc.light_count && !(target < cum[i + step - 1])) i += step;
+    found = target < cum[i];
+    if (!found) i = 0;
   }
-  if (pick < 0) {
-    float c = 0.f;
-    int last = -1;
-    for (uint32_t i = 0; i < sc.light_count; ++i) {
+  float c = 0.f;
+  int last = -1;
+  if (AREA == AREA_NONE && !found) {  // the weights alone are little work
+    for (; i < sc.light_count; ++i) {
       const float w = eval_light<AREA, HIT>(sc, lights, i, P, N, ev, wo_back, aop).w;
       c += w;
       if (w > 0.f) last = (int)i;
-      if (target < c) {
-        pick = (int)i;
-        break;
-      }
+      if (target < c) break;
     }
-    if (pick < 0) pick = last;
-    if (pick < 0) return false;
+    if (i == sc.light_count) {
+      if (last < 0) return false;
+      i = (uint32_t)last;
+    }
+    found = true;
   }
-  out = eval_light<AREA, HIT, BWD>(sc, lights, (uint32_t)pick, P, N, ev, wo_back, aop);
-  return true;
+  while (true) {
+    out = eval_light<AREA, HIT, BWD>(sc, lights, i, P, N, ev, wo_back, aop);
+    if (found) return true;
+    c += out.w;
+    if (out.w > 0.f) last = (int)i;
+    if (target < c) return true;
+    if (++i == sc.light_count) {
+      if (last < 0) return false;
+      i = (uint32_t)last;
+      found = true;
+    }
+  }
 }
 
 // Whether all of an area light's box lies clearly behind the plane through P
@@ -693,7 +707,7 @@ __device__ __forceinline__ int find_tile(const WaveArgs& a, int64_t x) {
 
 // ------------------------------------------------------------- generate --
 template <bool BWD, int AREA>
-__global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA ? kGenAreaBlocks : kGenBlocks)
+__global__ void __launch_bounds__(kThreads, BWD ? kAdjointBlocks : AREA == AREA_PAIRS ? kGenPairBlocks : kGenBlocks)
     k_generate(WaveArgs a) {
   extern __shared__ float dyn_smem[];
   const DLight* wave_lights = BWD ? nullptr : stage_lights(a.bakes, a.one_bake, reinterpret_cast<DLight*>(dyn_smem));
