@@ -737,12 +737,12 @@ void launch_shadow(cudaStream_t st, int grid, const BvhView* one, const BakeItem
 
 void launch_closest_rays(cudaStream_t st, int grid, const BvhView& bvh, const shb_ray* rays, int64_t n, float4* hits,
                          int* fetch, int* err) {
-  // The queue counter runs past the end by up to one ray per lane: chunks of
-  // 2^30 rays keep it within an int.
+  // The queue counter (cleared by the caller) runs past the end by up to one
+  // ray per lane: chunks of 2^30 rays keep it within an int.
   constexpr int64_t kChunk = int64_t(1) << 30;
   for (int64_t i = 0; i < n; i += kChunk) {
     const int m = (int)(n - i < kChunk ? n - i : kChunk);
-    cudaMemsetAsync(fetch, 0, sizeof(int), st);
+    if (i > 0) cudaMemsetAsync(fetch, 0, sizeof(int), st);
     const int need = (m + kTravThreads - 1) / kTravThreads;
     k_closest_rays<<<need < grid ? need : grid, kTravThreads, 0, st>>>(bvh, rays + i, m, hits + i, fetch, err);
   }
