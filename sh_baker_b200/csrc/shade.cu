@@ -330,7 +330,7 @@ __device__ __forceinline__ bool pick_light(const SceneView& sc, const DLight* li
   }
   float c = 0.f;
   int last = -1;
-  if (AREA == AREA_NONE && !found) {  // the weights alone are little work
+  if ((AREA == AREA_NONE || BWD) && !found) {  // the weights alone are less work (BWD: without the derivatives)
     for (; i < sc.light_count; ++i) {
       const float w = eval_light<AREA, HIT>(sc, lights, i, P, N, ev, wo_back, aop).w;
       c += w;
@@ -1457,7 +1457,7 @@ shb_status find_occlusion_device(shb_scene* s, const shb_ray* d_rays, int64_t n,
   SHB_TRY(c->scratch[9].reserve(sizeof(float4) * (size_t)n));
   SHB_TRY(c->counters.reserve(sizeof(int) * kCounterInts));
   int* cnt = c->counters.as<int>();
-  SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_DEPTH0, c->stream));
+  SHB_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (CNT_DEPTH0 + DC_COUNT), c->stream));
   float4* hits = c->scratch[9].as<float4>();
   launch_closest_rays(c->stream, traversal_grid(c->device, false), s->bvh(), d_rays, n, hits,
                       cnt + depth_cnt(0, DC_FETCH_EXT), cnt + CNT_ERROR);
